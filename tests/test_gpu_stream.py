@@ -128,3 +128,30 @@ def test_planes_with_an_outlier_in_every_run(wq, shape, tokens, dtype):
         exact = (x.double() @ (w.double() * sw.double()[:, None]).T + bias.double())
         assert rel(y, exact.float()) < 4e-3  # the output's own rounding to 8 or 11 bits
     assert wq.debug_status() == 0
+
+
+@pytest.mark.parametrize("entry,m", [("gemv_lines", 1), ("gemv_lines", 4), ("small", 8), ("small", 9), ("small", 16), ("small", 29)])
+def test_weights_straight_from_the_quantizer(wq, entry, m):
+    """The few-token kernels request weights before their digits are ready: codes that the kernel right before the call writes have to be the ones
+    that are used.  The buffers are the same ones over and over, with the opposite codes in them each time."""
+    n, k = 6144, 4096
+    g = torch.Generator(device="cuda").manual_seed(m)
+    x = torch.randn(m, k, device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn(n, k, device="cuda", generator=g).to(torch.bfloat16)
+    weights, call = (w, -w), getattr(wq, entry)
+    expected = []
+    for source in weights:
+        codes, _, scale = wq.quantize(source)
+        torch.cuda.synchronize()
+        expected.append(call(x, codes, scale))
+        torch.cuda.synchronize()
+    assert float((expected[0].float() + expected[1].float()).norm()) < 1e-3 * float(expected[0].float().norm())
+    del codes, scale
+    got = []
+    for i in range(20):
+        codes, _, scale = wq.quantize(weights[i % 2])
+        got.append(call(x, codes, scale))
+        del codes, scale  # the next round's codes go where these are
+    for i, y in enumerate(got):
+        assert torch.equal(y, expected[i % 2])
+    assert wq.debug_status() == 0

@@ -210,6 +210,12 @@ template <int GROUP> __host__ __device__ constexpr float group_norm() { return G
 // previous kernel has finished and its writes are visible.  The previous kernel lets the next one start early with dependents_may_start();
 // without it the next one starts when the previous one ends, as usual.  Data the previous kernel wrote is read with ordinary loads (below),
 // never through the read-only path, whose contract is that nobody writes the data while the kernel runs.
+//
+// A kernel launched this way calls dependency_wait() BEFORE dependents_may_start().  Otherwise the kernel behind it starts while kernels two
+// and more back are still running, and what it requests ahead of its own wait -- the few-token kernels their first weights -- may be what one
+// of those is writing (weight codes straight from a quantizer, which lets its dependents start as well).  In this order everything before
+// the previous kernel has finished when a kernel starts, so data that the previous kernel does not write may be requested at once.  A kernel
+// launched in the ordinary way starts after everything before it, and may let its dependents start first thing.
 WQ_DEVICE void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 WQ_DEVICE void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 WQ_DEVICE uint4 load_16(const void* p) {

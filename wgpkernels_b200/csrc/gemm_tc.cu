@@ -945,8 +945,8 @@ static bool make_output_map(CUtensorMap* map, const void* base, int m, int n, in
 // Weight scales of group-scaled weights, (N, kblocks) as the caller holds them -> (kblocks, n_pad) with zeros past N, so that the scales
 // a tile needs for one block of K are one contiguous run.
 __global__ void regroup_weight_scales(const float* sb, float* out, int n, int kblocks, int n_pad) {
-    dependents_may_start();
     dependency_wait();  // the workspace may be memory that the kernel before this one still reads
+    dependents_may_start();
     const int64_t total = int64_t(kblocks) * n_pad;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x) {
         const int kb = int(i / n_pad), col = int(i % n_pad);

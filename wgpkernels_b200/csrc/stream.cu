@@ -418,10 +418,10 @@ constexpr int kPlaneTokens = 8;  // token slots of the planes (one MMA column bl
 template <class T>
 __global__ void __launch_bounds__(256) split_planes(const T* x, int64_t ldx, int8_t* __restrict__ planes, float* __restrict__ scales, int m,
                                                     int k) {
-    // the stream kernel behind this one may start (its set-up and its first weight requests do not depend on the planes); this kernel
-    // itself may have started under the tail of the one that produced x
-    dependents_may_start();
+    // this kernel may have started under the tail of the one that produced x; once that has finished (it may have written the weights), the
+    // stream kernel behind this one may start: its set-up and its first weight requests do not depend on the planes
     dependency_wait();
+    dependents_may_start();
     const int lane = threadIdx.x & 31, runs = k / kPlaneRun;
     const int unit = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (unit >= runs * kPlaneTokens) return;

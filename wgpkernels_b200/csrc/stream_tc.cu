@@ -52,10 +52,11 @@ template <int TB> struct TcShape {
 // of (run, token), 0 for empty slots.  One warp per (token slot, run), 4 values per lane.
 template <class T, int TB>
 __global__ void __launch_bounds__(256) split_digits(const T* x, int64_t ldx, int8_t* __restrict__ digits, float* __restrict__ scales, int m, int k) {
-    // the stream kernel that follows may start (its set-up and its first weight loads do not depend on the digits); it waits for this
-    // grid to finish before it touches them.  This kernel itself may have started under the tail of the one that produced x.
-    dependents_may_start();
+    // This kernel may have started under the tail of the one that produced x.  Once that has finished, the stream kernel that follows may
+    // start (its set-up and its first weight loads do not depend on the digits; the weights themselves may come from the kernel waited for
+    // here); it waits for this grid to finish before it touches the digits.
     dependency_wait();
+    dependents_may_start();
     const int lane = threadIdx.x & 31, runs = k / kTcRun;
     const int unit = blockIdx.x * 8 + (threadIdx.x >> 5);
     constexpr int kRows = TcShape<TB>::kDigitRows, kSlots = kRows == 3 * TB ? TB : kRows - 2 * TB;  // TB = 8: 16 slots cover the padding rows
