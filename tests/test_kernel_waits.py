@@ -1,0 +1,53 @@
+"""The tensor-core kernels' bounded waits in their source (no GPU): what has to hold so that a wait that gives up ends the CTA and hangs nothing."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parents[1] / "wgpkernels_b200" / "csrc"
+TENSOR_CORE = ("gemm_tc.cu", "stream_tc.cu")
+
+
+def code(name):
+    return re.sub(r"//[^\n]*", "", (CSRC / name).read_text())
+
+
+@pytest.mark.parametrize("name", TENSOR_CORE)
+def test_no_lane_leaves_on_its_own(name):
+    """A wait is one lane's answer, and no lane leaves by it.  It goes through the warp's vote, or only the issuing lane waits and the warp votes
+    afterwards, or the lane that gave up keeps coming to the warp's meetings, or the answer is kept: for the vote behind it, or (sixteen drain
+    warps) for the abort flag's behind the tile."""
+    text = code(name)
+    waits = list(re.finditer(r"(?<!\w)(?:wait_on|tc_wait)\((?!uint32_t bar, uint32_t parity)", text))
+    assert len(waits) >= 4
+    for wait in waits:
+        before = re.split(r"[;{}]", text[:wait.start()])[-1]
+        behind = text[wait.start():].split("\n")[0]
+        assert "whole_warp(" in before or re.search(r"\bif \(leader && \(ok = ", before) or re.search(r"^\s*(?:const bool ready|ok) = ", before) or \
+            behind.endswith("{ left = steps_from(t, kb); break; }"), before
+    assert text.count("left = steps_from") == 2 * text.count("keep_meeting(left);") and len(re.findall(r"break; }\n\s*__syncwarp\(\);", text)) == text.count("keep_meeting(left);")
+    assert text.count("whole_warp(") >= 3
+
+
+def test_drains_that_go_on_leave_by_the_abort_flag():
+    text = code("gemm_tc.cu")
+    assert "if (!whole_warp(ready)) return false;" in text and "if (PARTS == 4) ok = whole_warp(*abort_flag == 0);" in text
+
+
+def test_streaming_waits_vote_at_the_call():
+    text = code("stream.cu")
+    waits = len(re.findall(r"(?<!\w)bulk_wait\(", text)) - 1  # (one is the definition)
+    assert waits > 0 and waits == len(re.findall(r"__all_sync\(0xffffffffu, bulk_wait\(", text))
+
+
+@pytest.mark.parametrize("name", TENSOR_CORE)
+def test_aborting_producers_wait_for_the_copies_they_issued(name):
+    """Asking for either parity of a barrier is no wait: one of them has always passed."""
+    assert "await_issued_fills(bar_full, kStages" in code(name) and "mbar_try_wait(" not in code(name)
+
+
+def test_warps_that_meet_at_a_named_barrier_agree_there():
+    """The drain warps of the few-token kernel meet once per shared tile; a warp that gave up has to come there as well."""
+    text = code("stream_tc.cu")
+    assert text.index("drains_agree(ok)") < text.index('"bar.sync 1, 128;"')
+    assert "drains_agree(false)" in text

@@ -44,6 +44,7 @@ constexpr long long kWaitLimit = 4000000000ll;  // clocks (about two seconds) be
 
 __device__ int g_status = 0;  // first code of a wait that gave up (wq::Status)
 
+// one lane's answer: to be put through whole_warp() before the warp acts on it
 WQ_DEVICE bool wait_on(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
     return mbar_wait(bar, parity, abort_flag, code, &g_status, kWaitLimit);
 }
@@ -283,7 +284,7 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                 const uint32_t bytes = tail ? uint32_t(p.tail_rows * kStageK * (S::kHilo ? 2 : 1) + S::kBBytes) : uint32_t(S::kStageBytes);
                 const int a_row = int(in_shift) + c.m0;
                 for (int kb = 0; kb < kblocks; ++kb) {
-                    if (!(ok = wait_on(bar_empty + 8 * stage, ((phases >> stage) & 1u) ^ 1u, abort_flag, kTimeoutEmpty))) break;
+                    if (!(ok = whole_warp(wait_on(bar_empty + 8 * stage, ((phases >> stage) & 1u) ^ 1u, abort_flag, kTimeoutEmpty)))) break;
                     phases ^= 1u << stage;
                     const uint32_t full = bar_full + 8 * stage;
                     const uint32_t dst = smem_u32(smem + stage * S::kStageBytes);
@@ -297,7 +298,6 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                             tma_load_2d_pair(dst + S::kABytes * (S::kHilo ? 2 : 1), &w_maps.map[c.segment], leader_full, kb * kStageK, c.n0 + int(rank) * (BN / 2));
                         }
                         if (++stage == kStages) stage = 0;
-                        __syncwarp();
                         continue;
                     }
                     if (leader) {
@@ -307,15 +307,16 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                         tma_load_2d(dst + S::kABytes * (S::kHilo ? 2 : 1), &w_maps.map[c.segment], full, kb * kStageK, c.n0);
                     }
                     if (++stage == kStages) stage = 0;
-                    __syncwarp();  // no lane falls behind the one that issues by a whole phase of a barrier
                 }
                 if (S::kStagePerIssuer && (kblocks & 1) && ++stage == kStages) stage = 0;  // the next tile starts on the first issuer's stages again
             }
             if (!ok) {
-                // aborting: let the copies already issued land before the CTA's shared memory is given back
-                for (int s = 0; s < kStages; ++s) {
+                // A pair's bytes are counted on the leader's barriers: the leader waits for both CTAs' copies, the other CTA for the leader (at
+                // the cluster barrier below).  A fill that only one of them has issued never completes its phase: time to land instead.
+                if (rank == 0) await_issued_fills(bar_full, kStages, phases);
+                if constexpr (PAIR) {
                     const long long start = clock64();
-                    while (!mbar_try_wait(bar_full + 8 * s, 0) && !mbar_try_wait(bar_full + 8 * s, 1) && clock64() - start < 2000000) {}
+                    while (clock64() - start < kLandLimit) {}
                 }
             }
         }
@@ -324,14 +325,15 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
         if (!S::kFold && rank == 0) {
             const bool leader = elect_one();
             constexpr uint32_t idesc = instruction_descriptor(BN, PAIR ? 2 * kBM : kBM);
-            int stage = 0, acc = 0;
+            int stage = 0, acc = 0, left = 0;
             uint32_t phase = 0, acc_phase = 0;
-            bool ok = true;
-            for (int t = tile_first; t < tiles && ok; t += tile_step) {
+            auto steps_from = [&](int t, int kb) { return kblocks - kb + (tiles - 1 - t) / tile_step * kblocks; };
+            for (int t = tile_first; t < tiles && !left; t += tile_step) {
                 for (int kb = 0; kb < kblocks; ++kb) {
                     const bool new_acc = kb == 0;
-                    if (new_acc && !(ok = wait_on(bar_acc_empty + 8 * acc, acc_phase ^ 1u, abort_flag, kTimeoutTmemEmpty))) break;
-                    if (!(ok = wait_on(bar_full + 8 * stage, phase, abort_flag, kTimeoutFull))) break;
+                    if (new_acc && !wait_on(bar_acc_empty + 8 * acc, acc_phase ^ 1u, abort_flag, kTimeoutTmemEmpty)) { left = steps_from(t, kb); break; }
+                    if (!wait_on(bar_full + 8 * stage, phase, abort_flag, kTimeoutFull)) { left = steps_from(t, kb); break; }
+                    __syncwarp();
                     tc_fence_after();
                     const uint32_t a_addr = smem_u32(smem + stage * S::kStageBytes);
                     const uint64_t a_desc = smem_descriptor(a_addr), a_lo_desc = smem_descriptor(a_addr + S::kABytes),
@@ -348,13 +350,13 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                         commit(bar_empty + 8 * stage);  // the stage may be refilled once these MMAs have read it
                         if (kb == kblocks - 1) commit(bar_acc_full + 8 * acc);
                     }
-                    __syncwarp();
                     if (++stage == kStages) { stage = 0; phase ^= 1u; }
                     if (kb == kblocks - 1) {
                         if (++acc == kAccBuffers) { acc = 0; acc_phase ^= 1u; }
                     }
                 }
             }
+            keep_meeting(left);
         }
     }
     if (S::kFold && (warp == 1 || warp == 2)) {
@@ -372,19 +374,21 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
             int stage = me % kStages;
             uint32_t phase = 0, buffer_phases = 0;  // of the stage in hand; bit b: phase of buffer b's next use
             uint32_t stage_phases = 0;              // a fixed issuer per stage: bit s = phase of stage s's next use
-            bool ok = true;
-            for (int t = tile_first; t < tiles && ok; t += tile_step) {
+            int left = 0;
+            auto steps_from = [&](int t, int kb) { return (kblocks - kb + 1) / 2 + (tiles - 1 - t) / tile_step * ((kblocks - me + 1) / 2); };
+            for (int t = tile_first; t < tiles && !left; t += tile_step) {
                 int kb = me;
                 for (; kb < kblocks; kb += 2) {
                     const int acc = kb % kAccBuffers;
                     const uint32_t d = tmem_base + acc * S::kAccColumns;
-                    if (!(ok = wait_on(bar_acc_empty + 8 * acc, ((buffer_phases >> acc) & 1u) ^ 1u, abort_flag, kTimeoutTmemEmpty))) break;
+                    if (!wait_on(bar_acc_empty + 8 * acc, ((buffer_phases >> acc) & 1u) ^ 1u, abort_flag, kTimeoutTmemEmpty)) { left = steps_from(t, kb); break; }
                     buffer_phases ^= 1u << acc;
                     if (S::kStagePerIssuer) {
                         phase = (stage_phases >> stage) & 1u;
                         stage_phases ^= 1u << stage;
                     }
-                    if (!(ok = wait_on(bar_full + 8 * stage, phase, abort_flag, kTimeoutFull))) break;
+                    if (!wait_on(bar_full + 8 * stage, phase, abort_flag, kTimeoutFull)) { left = steps_from(t, kb); break; }
+                    __syncwarp();
                     tc_fence_after();
                     const uint32_t a_addr = smem_u32(smem + stage * S::kStageBytes);
                     const uint64_t a_desc = smem_descriptor(a_addr), a_lo_desc = smem_descriptor(a_addr + S::kABytes),
@@ -400,7 +404,6 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                         commit(bar_empty + 8 * stage);
                         commit(bar_acc_full + 8 * acc);
                     }
-                    __syncwarp();
                     stage += 2;  // at most one wrap per step (kStages >= 2)
                     if (stage >= kStages) { stage -= kStages; phase ^= 1u; }
                 }
@@ -410,6 +413,7 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                 if (stage >= kStages) { stage -= kStages; phase ^= 1u; }
                 if (stage < 0) { stage += kStages; phase ^= 1u; }
             }
+            keep_meeting(left);
         }
     }
     if (warp == 3) {
@@ -425,7 +429,7 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
             auto stage_params = [&](const TileCoord& c) -> bool {
                 if (!p.vector_io) return true;
                 // every drain warp is done with the previous tile's parameters
-                if (tile_count > 0 && !wait_on(bar_params_consumed, uint32_t(tile_count - 1) & 1u, abort_flag, kTimeoutParams)) return false;
+                if (tile_count > 0 && !whole_warp(wait_on(bar_params_consumed, uint32_t(tile_count - 1) & 1u, abort_flag, kTimeoutParams))) return false;
                 const float* sb = p.sb[c.segment];
                 const T* bias = static_cast<const T*>(p.bias[c.segment]);
                 for (int i = lane; i < BN; i += 32) {
@@ -445,7 +449,7 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                     // the first two blocks' scales go first: the drain warps start on them right after the previous tile's write-out
                     const int params_after = (kblocks < 2 ? kblocks : 2) - 1;
                     for (int kb = 0; kb < kblocks && ok; ++kb) {
-                        if (!(ok = wait_on(bar_ring_empty + 8 * slot, phase ^ 1u, abort_flag, kTimeoutScales))) break;
+                        if (!(ok = whole_warp(wait_on(bar_ring_empty + 8 * slot, phase ^ 1u, abort_flag, kTimeoutScales)))) break;
                         // the tile's BN scales of this block are contiguous in sb_blocks: one bulk copy, up to kScaleRing of them in flight
                         if (lane == 0) {
                             mbar_expect_tx(bar_ring_full + 8 * slot, BN * 4);
@@ -454,7 +458,6 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                                          "l"(p.sb_blocks + int64_t(kb) * p.n_pad + c.n0), "r"(BN * 4), "r"(bar_ring_full + 8 * slot)
                                          : "memory");
                         }
-                        __syncwarp();
                         if (++slot == kScaleRing) { slot = 0; phase ^= 1u; }
                         if (kb == params_after) ok = stage_params(c);
                     }
@@ -492,7 +495,7 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
             // The tile's column parameters arrive in shared memory from warp 3; false when the CTA aborts.
             auto await_params = [&]() -> bool {
                 if (!p.vector_io) return true;
-                return __all_sync(0xffffffffu, wait_on(bar_params_written, uint32_t(tile_count) & 1u, abort_flag, kTimeoutParams));
+                return whole_warp(wait_on(bar_params_written, uint32_t(tile_count) & 1u, abort_flag, kTimeoutParams));
             };
             auto params_done = [&]() {
                 if (!p.vector_io) return;
@@ -704,10 +707,14 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                     if constexpr (S::kBlockScales && !DUMP) {
                         if (kb + 2 < kblocks) sa_after = sa_row[kb + 2];
                     }
-                    if constexpr (S::kWGroup) {
-                        if (!wait_on(bar_ring_full + 8 * slot, ring_phase, abort_flag, kTimeoutScales)) return false;
+                    // Sixteen drain warps: a vote here costs up to 7 % (16384 x 5120 x 13824: 1132 -> 1218 us).  A wait that gives up has raised the
+                    // CTA's abort flag and goes on without effect, as all the later ones then do at once; the warp leaves as one after the
+                    // tile's last block.  Eight drain warps are faster with the vote (1213 -> 1157 us).
+                    const bool ready = (!S::kWGroup || wait_on(bar_ring_full + 8 * slot, ring_phase, abort_flag, kTimeoutScales)) &
+                                       wait_on(bar_acc_full + 8 * BUFFER, (buffer_phases >> BUFFER) & 1u, abort_flag, kTimeoutTmemFull);
+                    if constexpr (PARTS == 2) {
+                        if (!whole_warp(ready)) return false;
                     }
-                    if (!wait_on(bar_acc_full + 8 * BUFFER, (buffer_phases >> BUFFER) & 1u, abort_flag, kTimeoutTmemFull)) return false;
                     buffer_phases ^= 1u << BUFFER;
                     tc_fence_after();
                     const uint32_t taddr = tmem_base + lane_base + BUFFER * S::kAccColumns + part * kEpi;
@@ -794,15 +801,20 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                     }
                     sa_now = sa_next;
                     sa_next = sa_after;
+                    // the block's sums are finished here: moved behind the next block's wait they would need more registers than there are
+#pragma unroll
+                    for (int j = 0; j < kEpi / 2; ++j) asm volatile("" : "+f"(accf[j].x), "+f"(accf[j].y));
                     return true;
                 };
                 // block kb of the tile uses buffer kb % kAccBuffers (the MMA issuers follow the same rule)
+#pragma unroll 1
                 for (int kb = 0; kb < kblocks && ok; kb += kAccBuffers) {
                     ok = drain_block(std::integral_constant<int, 0>(), kb);
                     if constexpr (kAccBuffers > 1) if (ok && kb + 1 < kblocks) ok = drain_block(std::integral_constant<int, 1>(), kb + 1);
                     if constexpr (kAccBuffers > 2) if (ok && kb + 2 < kblocks) ok = drain_block(std::integral_constant<int, 2>(), kb + 2);
                     if constexpr (kAccBuffers > 3) if (ok && kb + 3 < kblocks) ok = drain_block(std::integral_constant<int, 3>(), kb + 3);
                 }
+                if (PARTS == 4) ok = whole_warp(*abort_flag == 0);
                 if (!ok) break;
                 const int t_next = t + tile_step;
                 if (t_next < tiles) c_next = tile_at(t_next);
@@ -847,7 +859,7 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                     params_done();
                 }
             } else {
-                if (!(ok = __all_sync(0xffffffffu, wait_on(bar_acc_full + 8 * acc, acc_phase, abort_flag, kTimeoutTmemFull)))) break;
+                if (!(ok = whole_warp(wait_on(bar_acc_full + 8 * acc, acc_phase, abort_flag, kTimeoutTmemFull)))) break;
                 tc_fence_after();
                 const uint32_t taddr = tmem_base + lane_base + acc * S::kAccColumns + part * kEpi;
                 if (t + tile_step < tiles) c_next = tile_at(t + tile_step);
@@ -1280,8 +1292,15 @@ __global__ void bounded_wait_probe(long long clocks, int code, int* returned) {
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    const bool completed = mbar_wait(smem_u32(&bar), 0, &abort_word, code, &g_status, clocks);
-    if (threadIdx.x == 0) *returned = completed ? 1 : 2;
+    // every other lane asks for a phase that has passed: its warp gives up with it all the same
+    const unsigned completed = __ballot_sync(0xffffffffu, whole_warp(mbar_wait(smem_u32(&bar), threadIdx.x & 1u, &abort_word, code, &g_status, clocks)));
+    // what an aborting producer does: at once past a stage without a fill, and the whole limit for a fill that has not landed
+    const long long start = clock64();
+    await_issued_fills(smem_u32(&bar), 1, 0u);
+    const long long none = clock64();
+    await_issued_fills(smem_u32(&bar), 1, 1u);
+    const bool landing = none - start < kLandLimit && clock64() - none >= kLandLimit;
+    if (threadIdx.x == 0) *returned = completed ? 1 : landing ? 2 : 3;
 }
 }  // namespace wq
 

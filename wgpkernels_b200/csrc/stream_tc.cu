@@ -109,8 +109,23 @@ struct TcParams {
     int m, n, k, tiles, kblocks;
 };
 
+// one lane's answer: to be put through whole_warp() before the warp acts on it
 WQ_DEVICE bool tc_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
     return mbar_wait(bar, parity, abort_flag, 2, &g_tc_status, kTcWaitLimit);
+}
+
+// The four drain warps meet: do all of them go on?  (One that gave up comes here too, or the others would wait for it for ever.)
+WQ_DEVICE bool drains_agree(bool ok) {
+    uint32_t all;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.and.pred q, 1, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(all)
+        : "r"(uint32_t(ok))
+        : "memory");
+    return all != 0;
 }
 
 // start of CTA c's share of the `total` (tile, K block) pairs among `ctas`
@@ -171,7 +186,6 @@ stream_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
         {
             const bool leader = elect_one();
             int stage = 0;
-            uint32_t phase = 0;
             bool ok = true;
             // the ring's first fill: the weights go out at once, the digits of the same stages once the split has finished
             const long long first_fill = end - begin < kStages ? end - begin : kStages;
@@ -188,25 +202,20 @@ stream_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
                 const int kb = int((begin + i) % p.kblocks);
                 if (leader) tma_load_2d(smem_u32(smem + int(i) * S::kStageBytes) + S::kWeightBytes, &map_d, bar_full + 8 * int(i), kb * kTcRun, 0);
             }
-            if (first_fill == kStages) phase = 1u; else stage = int(first_fill);
+            uint32_t fills = (1u << int(first_fill)) - 1u;  // bit s: parity of the number of fills of stage s
             for (long long pair = begin + first_fill; pair < end && ok; ++pair) {
                 const int tile = int(pair / p.kblocks), kb = int(pair - (long long)tile * p.kblocks);
-                if (!(ok = tc_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag))) break;
                 const uint32_t full = bar_full + 8 * stage, dst = smem_u32(smem + stage * S::kStageBytes);
-                if (leader) {
+                if (leader && (ok = tc_wait(bar_empty + 8 * stage, ((fills >> stage) & 1u) ^ 1u, abort_flag))) {
                     mbar_expect_tx(full, S::kStageBytes);
                     tma_load_2d(dst, &map_w, full, kb * kTcRun, tile * kTcChannels);
                     tma_load_2d(dst + S::kWeightBytes, &map_d, full, kb * kTcRun, 0);
                 }
-                __syncwarp();  // no lane falls behind the one that issues by a whole phase of a barrier
-                if (++stage == kStages) { stage = 0; phase ^= 1u; }
+                if (!(ok = whole_warp(ok))) break;
+                fills ^= 1u << stage;
+                if (++stage == kStages) stage = 0;
             }
-            if (!ok) {
-                for (int s = 0; s < kStages; ++s) {  // aborting: let the copies already issued land before shared memory is given back
-                    const long long start = clock64();
-                    while (!mbar_try_wait(bar_full + 8 * s, 0) && !mbar_try_wait(bar_full + 8 * s, 1) && clock64() - start < 2000000) {}
-                }
-            }
+            if (!ok) await_issued_fills(bar_full, kStages, fills);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer: every K block is a fresh sum in the next accumulator buffer ----------------
@@ -217,12 +226,12 @@ stream_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
             uint32_t phase = 0;
             for (long long pair = begin, block = 0; pair < end; ++pair, ++block) {
                 const int acc = int(block % kAcc);
-                if (!tc_wait(bar_acc_empty + 8 * acc, (uint32_t(block / kAcc) & 1u) ^ 1u, abort_flag)) break;
-                if (!tc_wait(bar_full + 8 * stage, phase, abort_flag)) break;
-                tc_fence_after();
                 const uint32_t w_addr = smem_u32(smem + stage * S::kStageBytes);
                 const uint64_t w_desc = smem_descriptor(w_addr), d_desc = smem_descriptor(w_addr + S::kWeightBytes);
-                if (leader) {
+                bool ok = true;
+                if (leader && (ok = tc_wait(bar_acc_empty + 8 * acc, (uint32_t(block / kAcc) & 1u) ^ 1u, abort_flag) &&
+                                    tc_wait(bar_full + 8 * stage, phase, abort_flag))) {
+                    tc_fence_after();
 #pragma unroll
                     for (int j = 0; j < kTcRun / kMmaK; ++j) {
                         const uint64_t step = uint64_t(j * kMmaK >> 4);
@@ -231,7 +240,7 @@ stream_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
                     tc_commit(bar_empty + 8 * stage);
                     tc_commit(bar_acc_full + 8 * acc);
                 }
-                __syncwarp();
+                if (!whole_warp(ok)) break;
                 if (++stage == kStages) { stage = 0; phase ^= 1u; }
             }
         }
@@ -267,7 +276,7 @@ stream_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
                     scale4[i] = make_float4(__uint_as_float(bits.x), __uint_as_float(bits.y), __uint_as_float(bits.z), __uint_as_float(bits.w));
                 }
                 const int buffer = int(block % kAcc);
-                if (!(ok = tc_wait(bar_acc_full + 8 * buffer, uint32_t(block / kAcc) & 1u, abort_flag))) break;
+                ok = tc_wait(bar_acc_full + 8 * buffer, uint32_t(block / kAcc) & 1u, abort_flag);
                 tc_fence_after();
                 const uint32_t taddr = tmem_base + lane_base + buffer * N;
                 int sums[3][TB];
@@ -281,7 +290,7 @@ stream_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
 #pragma unroll
                 for (int plane = 0; plane < 3; ++plane) tmem_loaded(sums[plane]);
                 tc_fence_before();
-                __syncwarp();
+                if (!(ok = whole_warp(ok))) break;
                 if (lane == 0) mbar_arrive(bar_acc_empty + 8 * buffer);  // the sums are in registers: the buffer goes back to the MMAs
                 const float* scale = reinterpret_cast<const float*>(scale4);
 #pragma unroll
@@ -291,9 +300,13 @@ stream_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
                     acc[t] = fmaf(combined, scale[t], acc[t]);
                 }
             }
-            if (!ok) break;
             const bool whole = kb0 == 0 && kb1 == p.kblocks;
             bool finish = whole;
+            if (whole && !ok) {
+                // the other warps may still come to the piece that the share ends with, if it ends with one
+                if (end % p.kblocks != 0) drains_agree(false);
+                break;
+            }
             if (!whole) {
                 // a piece of a tile: into this CTA's slot (0: the tile its share starts in, 1: the tile it ends in), then the tile's counter
                 const int which = (long long)tile * p.kblocks <= begin ? 0 : 1;
@@ -301,7 +314,7 @@ stream_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
 #pragma unroll
                 for (int t = 0; t < TB; ++t) __stcg(slot + t * kTcChannels + thread, acc[t]);
                 __threadfence();
-                asm volatile("bar.sync 1, 128;" ::: "memory");  // the four drain warps
+                if (!(ok = drains_agree(ok))) break;
                 const long long first_pair = (long long)tile * p.kblocks;
                 const int first_cta = int(cta_of_pair(first_pair, total, ctas)), last_cta = int(cta_of_pair(first_pair + p.kblocks - 1, total, ctas));
                 if (thread == 0) arrival = atomicAdd(p.counters + tile, 1);

@@ -94,6 +94,29 @@ WQ_DEVICE bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag
     }
 }
 
+// A warp leaves a role as one.  Lanes that decided for themselves could part on an abort: one leaves for the CTA's last barrier, the others wait
+// for it wherever the warp meets next, for ever.  And every lane has looked at a phase before the warp acts on it: what is issued lets the
+// barrier go on, and a lane that looked a whole phase later would take its parity for one that has yet to complete.  So a role votes on a
+// wait (or, where only one lane waits, on what came of it),
+WQ_DEVICE bool whole_warp(bool ok) { return __all_sync(0xffffffffu, ok); }
+// or, where the vote costs too much (the MMA issuers: `exact` on 64 x 5120 x 5120 20.7 -> 21.8 us), the warp meets with __syncwarp() behind the
+// waits of every step, and a lane that gave up keeps coming to the meetings of the steps that are left.
+WQ_DEVICE void keep_meeting(int steps) {
+#pragma unroll 1
+    for (; steps > 0; --steps) __syncwarp();
+}
+
+// An aborting producer: waits for the last copies it issued into each of its stages, so that shared memory is not given back under them.
+// Bit s of `fills`: parity of the number of fills issued into stage s; the last one completes the phase of the opposite parity (on a barrier
+// without a fill that phase counts as completed).  At most kLandLimit clocks (a millisecond, against the microseconds of a copy) a stage.
+constexpr long long kLandLimit = 2000000;
+WQ_DEVICE void await_issued_fills(uint32_t bar_full, int stages, uint32_t fills) {
+    for (int s = 0; s < stages; ++s) {
+        const long long start = clock64();
+        while (!mbar_try_wait(bar_full + 8 * s, ((fills >> s) & 1u) ^ 1u) && clock64() - start < kLandLimit) {}
+    }
+}
+
 WQ_DEVICE void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst), "l"(map),
                  "r"(bar), "r"(x), "r"(y)
