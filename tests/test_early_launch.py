@@ -50,6 +50,13 @@ def test_waits_before_it_lets_the_next_one_start(name):
         assert body.index("dependency_wait()") < body.index("dependents_may_start()")
 
 
+@pytest.mark.parametrize("name", ["gemm_i8_tc", "regroup_weight_scales", "split_digits", "split_planes"])
+def test_reads_what_the_kernel_before_it_may_have_written_with_ordinary_loads(name):
+    """These start behind any kernel, a quantizer that wrote the weights and their scales included.  The read-only path is for data that nobody
+    writes while the kernel runs, and its loads may be moved ahead of the wait."""
+    assert not re.search(r"__ldg\(|(?<!\w)load_eight\(|ld\.global\.nc", BODIES[name])
+
+
 @pytest.mark.parametrize("name", sorted(n for n, body in BODIES.items() if "dependents_may_start()" in body))
 def test_lets_the_next_one_start_only_where_everything_before_it_has_finished(name):
     assert "dependency_wait()" in BODIES[name] or name not in launched_early()

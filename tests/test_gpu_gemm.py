@@ -327,3 +327,27 @@ def test_tile_shapes_agree(wq, mode, shape):
                           for v in SHAPES_OF[mode]]
         assert all(torch.equal(first, y) for y in others)
     assert wq.debug_status() == 0
+
+
+@pytest.mark.parametrize("mode", ["row", "block", "exact"])
+def test_weights_and_scales_straight_from_the_quantizer(wq, mode):
+    """The GEMM is launched under the tail of the kernel before it, here the quantizer of the weights themselves: codes and scales in the same
+    buffers over and over, with the opposite codes and twice the scales in them each time."""
+    m, n, k = 200, 4096, 1024
+    g = torch.Generator(device="cuda").manual_seed(7)
+    w = torch.randn(n, k, device="cuda", generator=g).to(torch.bfloat16)
+    prepared = wq.prepare(torch.randn(m, k, device="cuda", generator=g).to(torch.bfloat16), path=mode)
+    weights, expected = (w, -2 * w), []
+    for source in weights:
+        codes, _, scale = wq.quantize(source)
+        torch.cuda.synchronize()
+        expected.append(wq.linear_prepared(prepared, codes, scale))
+        torch.cuda.synchronize()
+    assert torch.equal(expected[1], -2 * expected[0])
+    del codes, scale
+    got = []
+    for i in range(20):
+        codes, _, scale = wq.quantize(weights[i % 2])
+        got.append(wq.linear_prepared(prepared, codes, scale))
+        del codes, scale  # the next round's codes go where these are
+    assert all(torch.equal(y, expected[i % 2]) for i, y in enumerate(got)) and wq.debug_status() == 0

@@ -239,17 +239,16 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
     const uint32_t tmem_base = tmem_slot;
 
     // Launched behind the kernel before it on the stream (programmatic stream serialization): the set-up above runs under the tail of the
-    // quantizer, everything below touches memory that it or an earlier kernel may have written (the activation scales are therefore
-    // read with ordinary loads, not through the read-only path).
+    // quantizer, everything below touches memory that it or an earlier kernel may have written (weights and scales straight from a
+    // quantizer among it), and is read with ordinary loads, not through the read-only path.
     dependency_wait();
     // row window of the *_at entry points: where the outputs go and where the inputs come from
     long long out_shift = 0, in_shift = 0;
     if (p.window.counter) {
-        const long long count = __ldg(p.window.counter);
+        const long long count = *p.window.counter;
         out_shift = p.window.first + count * p.window.step;
         if (p.window.in_first || p.window.in_step) in_shift = p.window.in_first + count * p.window.in_step;
     }
-
 
     auto issue_mma = [](uint32_t d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
         if constexpr (PAIR) mma_i8_pair(d, a_desc, b_desc, idesc, accumulate);
@@ -435,7 +434,7 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                 for (int i = lane; i < BN; i += 32) {
                     const int col = c.n0 + i;
                     const bool inside = col < p.n;
-                    param_sb[i] = !S::kWGroup && inside ? __ldg(sb + col) : 0.f;
+                    param_sb[i] = !S::kWGroup && inside ? sb[col] : 0.f;
                     param_bias[i] = bias && inside ? as_float(bias[col]) : 0.f;
                     param_rscale[i] = rscale && !p.window.span && inside ? rscale[col] : round_one<T>(1.f);
                 }
@@ -547,8 +546,7 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                         if (res) {
                             float res8[8], rs8[8];
                             load_eight_plain(res + j, res8);  // read before this thread overwrites it (y may be the residual)
-                            if (rs_row) load_eight(rs_row + col + j, rs8, true);
-                            else load_eight_plain(param_rscale + ct, rs8);
+                            load_eight_plain(rs_row ? rs_row + col + j : param_rscale + ct, rs8);
 #pragma unroll
                             for (int e = 0; e < 8; ++e) out[e] = fmaf(out[e], rs8[e], res8[e]);
                         }
@@ -598,7 +596,7 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                     for (int j = 0; j < 16; ++j) {
                         const int cj = col + part16 + j;
                         if (row_ok && cj < p.n) {
-                            const float col_scale = S::kWGroup ? 1.f : __ldg(sb + cj);
+                            const float col_scale = S::kWGroup ? 1.f : sb[cj];
                             float value = fmaf(mine[j] * row_scale, col_scale, bias ? as_float(bias[cj]) : 0.f);
                             if (res) {
                                 const T* rs = rscale && p.window.span ? rscale + (out_shift + row) / p.window.span * p.window.scale_step : rscale;
