@@ -66,8 +66,8 @@ template <int MODE, int BN, bool WIDE, int PARTS, bool PAIR> struct Shape {
     static constexpr int kStageBytes = kABytes * (kHilo ? 2 : 1) + kBBytes;
     static constexpr int kEpiColumns = BN / PARTS;  // columns per drain thread (PARTS warps split the tile's columns)
     // Columns a drain thread brings in from tensor memory at once, into one of two staging sets.  Few enough that nothing spills while loads are
-    // in flight: a spilled staging register may be stored before its load has delivered it (block+g with eight drain warps lost columns that
-    // way, now and then, so it is not built any more).
+    // in flight: a spilled staging register may be stored before its load has delivered it (the build refuses kernels that spill; block+g
+    // with eight drain warps would).
     static constexpr int kChunk = PARTS == 2 ? 32 : kWGroup && BN == 256 ? 8 : 16;
     static_assert(!(kWGroup && PARTS == 2 && BN == 256), "block+g on 256 columns needs sixteen drain warps");
     static constexpr int kRingBytes = kWGroup ? kScaleRing * BN * 4 : 0;
@@ -614,6 +614,15 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
             // for the TMA unit to be done reading the staging tile of the previous chunk, so that wait hides behind the arithmetic.
             // Same operations per output, in the same order, as `emit`: the bits do not depend on which of the two writes a tile.
             const bool fast_tile = !S::kWide && p.vector_io && p.tma_y && p.destinations == 1 && c.n0 + BN <= p.n && !(rscale && p.window.span);
+            // 16-byte piece g of the 32 residual values that belong to chunk `chunk` of this thread's row (plain loads: y may be the residual).  For
+            // block+g on 256 channels a piece is fetched where it is added: four at once spill.
+            const T* res_row = residual && row_ok ? residual + (out_shift + row) * p.ld_residual + col0 : nullptr;
+            constexpr bool kResidualByPiece = MODE == kBlockG && BN == 256;
+            auto fetch_residual_piece = [&](int chunk, int g) { return *reinterpret_cast<const uint4*>(res_row + chunk * 32 + 8 * g); };
+            auto fetch_residual = [&](int chunk, uint4* res) {
+#pragma unroll
+                for (int g = 0; g < 4; ++g) res[g] = fetch_residual_piece(chunk, g);
+            };
             auto emit_fast = [&](const float2* a, int chunk, const uint4* res, bool has_res) {
                 const int ct = part * kEpi + chunk * 32;  // first column of the chunk within the tile
                 uint32_t packed[16];
@@ -638,8 +647,9 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                         }
                     }
                     if (has_res) {
+                        const uint4 res_g = kResidualByPiece ? fetch_residual_piece(chunk, g) : res[g];
                         const uint4 rs = *reinterpret_cast<const uint4*>(param_rscale + ct + 8 * g);
-                        const uint32_t rs_raw[4] = {rs.x, rs.y, rs.z, rs.w}, res_raw[4] = {res[g].x, res[g].y, res[g].z, res[g].w};
+                        const uint32_t rs_raw[4] = {rs.x, rs.y, rs.z, rs.w}, res_raw[4] = {res_g.x, res_g.y, res_g.z, res_g.w};
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
                             float2 scale2, res2;
@@ -670,12 +680,6 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                                  : "memory");
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 }
-            };
-            // 16-byte piece g of the 32 residual values that belong to chunk `chunk` of this thread's row (plain loads: y may be the residual)
-            const T* res_row = residual && row_ok ? residual + (out_shift + row) * p.ld_residual + col0 : nullptr;
-            auto fetch_residual = [&](int chunk, uint4* res) {
-#pragma unroll
-                for (int g = 0; g < 4; ++g) res[g] = *reinterpret_cast<const uint4*>(res_row + chunk * 32 + 8 * g);
             };
 
             if constexpr (S::kFold) {
@@ -839,7 +843,7 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                                 if (res_row && chunk + 1 < kEpi / 32) fetch_residual(chunk + 1, res[(chunk + 1) & 1]);
                                 emit_fast(&accf[chunk * 16], chunk, res[chunk & 1], res_row != nullptr);
                             } else {
-                                if (res_row) fetch_residual(chunk, res[0]);
+                                if (!kResidualByPiece && res_row) fetch_residual(chunk, res[0]);
                                 emit_fast(&accf[chunk * 16], chunk, res[0], res_row != nullptr);
                             }
                         }
