@@ -71,8 +71,9 @@ int wq8_gemm(const int8_t* a, const int8_t* a_lo, const float* sa, const int8_t*
              int* workspace, int* counters, wq8_stream_t stream);
 
 /* Addition without a reference counterpart: quantizer and wq8_gemm of one row band in one call.  path: 0 'block', 1 'exact', 2 'row', variant one
- * of that mode (by sw's layout); scratch: wq8_linear_scratch() bytes, 256-byte aligned, free again once the work on `stream` is done.
- * Codes: those of the two calls; -1 dtype, -2 K not a multiple of 16, path, scratch. */
+ * of that mode (by sw's layout); scratch: wq8_linear_scratch() bytes (0 for sizes, a path or a variant that wq8_linear refuses), 256-byte
+ * aligned, free again once the work on `stream` is done.  Codes: those of the two calls; before anything is launched -1 dtype, -2 K not a
+ * multiple of 16, path, a variant of another mode than the path's, scratch, -3 variant. */
 int64_t wq8_linear_scratch(int m, int n, int k, int path, int variant, int sms);
 int wq8_linear(const void* x, int64_t ldx, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale,
                void* y, int m, int n, int k, int dtype, int group, int act, const void* act_weight, float eps, int path, int variant,

@@ -172,3 +172,26 @@ def test_row_window_entry_points_check_their_arguments(lib):
     assert lib.wq8_quantize_at(None, None, None, None, 0, 256, 256, 1, 0, 0, None, 0.0, one, 0, 1, None) == 0
     assert lib.wq8_quantize_at(one, one, None, one, 4, 256, 256, 5, 0, 0, None, 0.0, one, 0, 1, None) == -1
     assert lib.wq8_quantize_blocks_at(one, one, one, 4, 250, 256, 1, 0, 0, None, 0.0, None, one, 0, 1, None) == -2
+
+
+def test_one_call_linear_checks_path_and_variant(lib):
+    """The quantizer of a path writes the scales that the variants of its mode read; another variant is refused before anything is launched."""
+    lib.wq8_linear_scratch.argtypes, lib.wq8_linear_scratch.restype = [i] * 6, i64
+    lib.wq8_linear.argtypes = [p, i64, p, p, p, p, p, p, i, i, i, i, i, i, p, f, i, i, i, p, p]
+    one, scratch = p(16), p(4096)
+    modes = {0: (10, 11, 12, 13, 15, 16, 17, 18, 20, 22), 1: (1, 7, 14, 19, 24, 37, 38), 2: (0, 2, 6, 30, 35, 36)}
+
+    def call(path, variant, dtype=1, k=256, scratch=scratch):
+        return lib.wq8_linear(one, 256, one, one, None, None, None, one, 8, 96, k, dtype, 0, 0, None, 0.0, path, variant, 148, scratch, None)
+
+    for path in modes:
+        for own, variants in modes.items():
+            for variant in variants:
+                size = lib.wq8_linear_scratch(8, 96, 256, path, variant, 148)
+                assert (size > 0) == (path == own), (path, variant)
+                if path != own:
+                    assert call(path, variant) == -2, (path, variant)
+        assert call(path, 99) == -3 and lib.wq8_linear_scratch(8, 96, 256, path, 99, 148) == 0
+    for path in (-1, 3):
+        assert call(path, 10) == -2 and lib.wq8_linear_scratch(8, 96, 256, path, 10, 148) == 0
+    assert call(0, 10, dtype=2) == -1 and call(0, 10, k=250) == -2 and call(0, 10, scratch=None) == -2 and call(0, 10, scratch=p(4096 + 128)) == -2

@@ -71,6 +71,7 @@ void wq8_gemm_workspace(int, int, int, int, int, int, int64_t*);
 }
 
 namespace wq {
+int path_and_variant(int path, int variant);  // gemm_tc.cu
 struct LinearScratch { int64_t codes, low, scales, workspace, total; };  // offsets of the parts, 256-byte aligned
 static LinearScratch linear_scratch(int m, int n, int k, int path, int variant, int sms) {
     auto padded = [](int64_t bytes) { return (bytes + 255) / 256 * 256; };
@@ -86,7 +87,7 @@ static LinearScratch linear_scratch(int m, int n, int k, int path, int variant, 
 }  // namespace wq
 
 WQ_API int64_t wq8_linear_scratch(int m, int n, int k, int path, int variant, int sms) {
-    if (m <= 0 || n <= 0 || k <= 0 || path < 0 || path > 2) return 0;
+    if (m <= 0 || n <= 0 || k <= 0 || wq::path_and_variant(path, variant)) return 0;
     return wq::linear_scratch(m, n, k, path, variant, sms).total;
 }
 
@@ -95,7 +96,8 @@ WQ_API int wq8_linear(const void* x, int64_t ldx, const int8_t* w, const float* 
                       void* scratch, cudaStream_t stream) {
     if (m <= 0 || n <= 0) return 0;
     if (dtype != 0 && dtype != 1) return -1;
-    if (k <= 0 || k % 16 || path < 0 || path > 2 || !scratch || (reinterpret_cast<uintptr_t>(scratch) & 255)) return -2;
+    if (const int code = wq::path_and_variant(path, variant)) return code;
+    if (k <= 0 || k % 16 || !scratch || (reinterpret_cast<uintptr_t>(scratch) & 255)) return -2;
     const wq::LinearScratch s = wq::linear_scratch(m, n, k, path, variant, sms);
     auto base = static_cast<int8_t*>(scratch);
     int8_t* low = path == 1 ? base + s.low : nullptr;

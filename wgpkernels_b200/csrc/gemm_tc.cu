@@ -1188,9 +1188,25 @@ template <class T> static int dispatch(const GemmArgs& g, int variant, cudaStrea
     return -3;
 }
 
-static bool takes_low_part(int variant) { return variant == 1 || variant == 7 || variant == 14 || variant == 19 || variant == 24 || variant == 37 || variant == 38; }
-static bool takes_group_scales(int variant) {
-    return (variant >= 12 && variant <= 14) || variant == 18 || variant == 19 || variant == 22 || variant == 24;
+// The Mode of a variant, -1 for a number that is none.
+static int mode_of(int variant) {
+    switch (variant) {
+        case 0: case 2: case 6: case 30: case 35: case 36: return kRow;
+        case 1: case 7: case 37: case 38: return kExact;
+        case 10: case 11: case 15: case 16: case 17: case 20: return kBlock;
+        case 12: case 13: case 18: case 22: return kBlockG;
+        case 14: case 19: case 24: return kExactG;
+    }
+    return -1;
+}
+static bool takes_low_part(int variant) { return mode_of(variant) == kExact || mode_of(variant) == kExactG; }
+static bool takes_group_scales(int variant) { return mode_of(variant) == kBlockG || mode_of(variant) == kExactG; }
+
+// wq8_linear: 0 when the quantizer of `path` (0 block, 1 exact, 2 row) writes what this variant reads, else the error code.
+int path_and_variant(int path, int variant) {
+    const int mode = mode_of(variant);
+    if (mode < 0) return -3;
+    return (path == 0 ? mode == kBlock || mode == kBlockG : path == 1 ? mode == kExact || mode == kExactG : path == 2 && mode == kRow) ? 0 : -2;
 }
 
 static int gemm_entry(GemmArgs& g, int dtype, int variant, cudaStream_t stream) {
