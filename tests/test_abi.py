@@ -195,3 +195,15 @@ def test_one_call_linear_checks_path_and_variant(lib):
     for path in (-1, 3):
         assert call(path, 10) == -2 and lib.wq8_linear_scratch(8, 96, 256, path, 10, 148) == 0
     assert call(0, 10, dtype=2) == -1 and call(0, 10, k=250) == -2 and call(0, 10, scratch=None) == -2 and call(0, 10, scratch=p(4096 + 128)) == -2
+
+
+def test_a_library_without_this_modules_additions_is_reported(tmp_path):
+    """An older build speaks the same ABI number and lacks entry points that were added since."""
+    from wgpkernels_b200 import int8
+    source, library = tmp_path / "old.c", tmp_path / "libold.so"
+    source.write_text("int wq8_abi(void) { return 11; }\nint wq8_features(void) { return 1; }\n")
+    subprocess.run(["gcc", "-shared", "-fPIC", str(source), "-o", str(library)], check=True)
+    loaded = int8._lib
+    with pytest.raises(RuntimeError, match="rebuild it"):
+        int8.load_library(library)
+    assert int8._lib is loaded
