@@ -318,7 +318,8 @@ SHAPES_OF = {"row": (2, 30, 35, 36, 0), "exact": (7, 37, 38, 1), "block": (20, 1
 @pytest.mark.parametrize("mode", sorted(SHAPES_OF))
 def test_tile_shapes_agree(wq, mode, shape):
     """Tiles of 64, 128 and 256 channels and pairs of CTAs give the same bits: INT32 sums are exact, and every output takes the same FP32 steps
-    in the same order.  Partial tiles in both directions, K shorter and longer than the stages, odd numbers of blocks, several tiles per CTA."""
+    in the same order.  Partial tiles in both directions, K shorter and longer than the stages, odd numbers of blocks; at most one tile per CTA of the wide shapes
+    (several: test_every_tile_shape_over_several_tiles)."""
     m, n, k = shape
     base, a, a_lo, sa, b, sb, bias, res, rs = operands(mode, m, n, k, torch.bfloat16, 600 + m, residual=True)
     a, a_lo, sa, b, sb, bias, res, rs = (None if t is None else t.cuda() for t in (a, a_lo, sa, b, sb, bias, res, rs))
@@ -351,3 +352,65 @@ def test_weights_and_scales_straight_from_the_quantizer(wq, mode):
         got.append(wq.linear_prepared(prepared, codes, scale))
         del codes, scale  # the next round's codes go where these are
     assert all(torch.equal(y, expected[i % 2]) for i, y in enumerate(got)) and wq.debug_status() == 0
+
+
+EVERY_SHAPE_OF = {"row": (2, 6, 30, 35, 36, 0), "exact": (7, 37, 38, 1), "block": (10, 11, 20, 16, 17, 15), "block+g": (12, 22, 18, 13), "exact+g": (24, 19, 14)}
+
+
+@pytest.mark.parametrize("blocks", [4, 5])
+@pytest.mark.parametrize("mode", sorted(EVERY_SHAPE_OF))
+def test_every_tile_shape_over_several_tiles(wq, mode, blocks):
+    """Three and more tiles per CTA, or per pair of CTAs, in every shape: buffers and stages that come round, parameters handed over from tile to
+    tile, partial tiles at both edges.  The first shape against the same sums in 64 bits (the rounding of the BF16 output is at most 2^-8 of a
+    value, half of that on average; FP32 sums are far closer), the others bit for bit against the first, with a residual in place too."""
+    m, n, k = 256 * 13 - 5, 256 * 20 + 8, 128 * blocks - 16
+    assert -(-m // 256) * -(-n // 256) > 3 * 74
+    base, a, a_lo, sa, b, sb, bias, res, rs = (t.cuda() if torch.is_tensor(t) else t for t in operands(mode, m, n, k, torch.bfloat16, 700 + blocks, residual=True))
+    exact = torch.zeros(m, n, dtype=torch.float64, device="cuda")
+    for i in range(blocks):
+        cut = slice(128 * i, min(128 * (i + 1), k))
+        sums = a[:, cut].double() @ b[:, cut].double().T
+        if a_lo is not None:
+            sums += a_lo[:, cut].double() @ b[:, cut].double().T / 254
+        exact += sums * (sa[:, i, None] if sa.dim() == 2 else sa[:, None]).double() * (sb[None, :, i] if sb.dim() == 2 else 1.0)
+    exact = (exact if sb.dim() == 2 else exact * sb[None, :].double()) + bias.double()
+    plain = added = None
+    for variant in EVERY_SHAPE_OF[mode]:
+        y = wq.gemm(a, a_lo, sa, b, sb, bias, torch.bfloat16, 0, variant)
+        out = res.clone()
+        wq.gemm(a, a_lo, sa, b, sb, bias, torch.bfloat16, 0, variant, out=out, residual=out, residual_scale=rs)
+        if plain is None:
+            plain, added = y, out
+            with_residual = res.double() + rs.double() * exact
+            assert float((y.double() - exact).norm() / exact.norm()) < 2.0 ** -8
+            assert float((out.double() - with_residual).norm() / with_residual.norm()) < 2.0 ** -8
+        assert torch.equal(y, plain) and torch.equal(out, added), variant
+    assert wq.debug_status() == 0
+
+
+def test_segments_on_pairs_of_ctas(wq):
+    """Segments wide enough for the row path's pairs of CTAs, several tiles per pair, column tiles that end inside a weight."""
+    m, rows, k, dtype = 256 * 13 - 5, 256 * 6 + 8, 640, torch.bfloat16
+    _, a, _, sa, b, sb, bias, _, _ = operands("row", m, 3 * rows, k, dtype, 92)
+    a, sa, b, sb, bias = (t.cuda() for t in (a, sa, b, sb, bias))
+    prepared = wq.Prepared("row", a, None, sa, dtype)
+    cut = lambda t, s: t[s * rows:(s + 1) * rows].contiguous()
+    weights, scales, biases = ([cut(t, s) for s in range(3)] for t in (b, sb, bias))
+    outputs = [torch.empty((m, rows), dtype=dtype, device="cuda") for _ in range(3)]
+    wq.linear_prepared_segments(prepared, weights, scales, biases, outputs)
+    for s, y in enumerate(outputs):
+        assert torch.equal(y, wq.gemm(a, None, sa, weights[s], scales[s], biases[s], dtype, 0, 2))
+    assert wq.debug_status() == 0
+
+
+@pytest.mark.parametrize("mode,variant", [("row", 2), ("row", 30), ("row", 35), ("exact", 7), ("exact", 37), ("block", 16), ("exact+g", 24), ("block+g", 18)])
+@pytest.mark.parametrize("shape", [(40, 96, 256), (130, 264, 640), (257, 520, 1024 + 48)], ids=str)
+def test_explicit_tile_shapes_match_oracle(wq, shape, mode, variant):
+    """The tile shapes that the rules would not choose for these sizes, against the oracle."""
+    m, n, k = shape
+    dtype = torch.float16
+    base, a, a_lo, sa, b, sb, bias, res, rs = operands(mode, m, n, k, dtype, 33, True)
+    dev = lambda t: None if t is None else t.cuda()
+    y = wq.gemm(dev(a), dev(a_lo), dev(sa), dev(b), dev(sb), dev(bias), dtype, 0, variant, residual=dev(res), residual_scale=dev(rs))
+    expected = oracle.gemm(base, a.numpy(), None if a_lo is None else a_lo.numpy(), sa.numpy(), b.numpy(), sb.numpy(), bias, res, rs, dtype)
+    assert rel(y, expected) < 1e-3 and wq.debug_status() == 0
