@@ -55,6 +55,8 @@ WQ_DEVICE bool wait_on(uint32_t bar, uint32_t parity, volatile int* abort_flag, 
 // the bits of 1.5 * 2^23, so that one FP32 subtraction converts, cost more than they save: re-arming a buffer from registers takes a
 // register move per column, on the FP32 pipe.)
 template <int MODE, int BN, bool WIDE, int PARTS, bool PAIR> struct Shape {
+    // (`exact` is at the power limit with single CTAs; in the per-block modes the hand-over of a buffer would cross the cluster)
+    static_assert(!PAIR || MODE == kRow, "pairs of CTAs are built for row only");
     static constexpr int kDrainWarps = Roles<PARTS>::kDrainWarps;
     static constexpr bool kHilo = MODE == kExact || MODE == kExactG;
     static constexpr bool kFold = MODE == kBlock || MODE == kBlockG || MODE == kExactG;  // one accumulation per 128 of K
@@ -99,7 +101,8 @@ template <int MODE, int BN, bool WIDE, int PARTS, bool PAIR> struct Shape {
     // barrier's parity test (one phase bit) for passed.  It cannot be that early: it has just got its buffer back, so the drain has
     // consumed the block that used the buffer last -- at most three blocks before, with two buffers --, and the operands of that block and
     // of every earlier one have landed.
-    static_assert(!kFold || kStages % 2 == 0 || (kStages >= 3 && kAccBuffers == 2), "an odd number of stages is safe with two issuers from three stages on, with two buffers");
+    static_assert(!kFold || kStages % 2 == 0 || (kStages >= 3 && kAccBuffers == 2),
+                  "an odd number of stages is safe with two issuers from three stages on, with two buffers");
     static_assert(kEpiColumns % 32 == 0, "a drain thread works on chunks of 16 or 32 and writes out chunks of 32 columns");
 };
 
@@ -293,8 +296,7 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                         if (leader) {
                             if (rank == 0) mbar_expect_tx(full, 2 * S::kStageBytes);
                             tma_load_2d_pair(dst, &in_maps.a, leader_full, kb * kStageK, c.m0);
-                            if (S::kHilo) tma_load_2d_pair(dst + S::kABytes, &in_maps.a_lo, leader_full, kb * kStageK, c.m0);
-                            tma_load_2d_pair(dst + S::kABytes * (S::kHilo ? 2 : 1), &w_maps.map[c.segment], leader_full, kb * kStageK, c.n0 + int(rank) * (BN / 2));
+                            tma_load_2d_pair(dst + S::kABytes, &w_maps.map[c.segment], leader_full, kb * kStageK, c.n0 + int(rank) * (BN / 2));
                         }
                         if (++stage == kStages) stage = 0;
                         continue;
@@ -363,10 +365,10 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
         // Block kb of a tile goes to accumulator buffer kb % kAccBuffers (2 buffers of 256 columns, or 4 of 128: the drain warps' loop
         // over the blocks is unrolled by the buffers, so every buffer has its own code there) and is issued by warp 1 + kb % 2, so that one
         // warp's barrier tests and commits overlap the other one's MMAs.
-        if (rank == 0) {
+        {
             const bool leader = elect_one();
             static_assert(!S::kFold || (kStages >= 2 && kAccBuffers % 2 == 0), "two issuers alternate over an even number of buffers");
-            constexpr uint32_t idesc = instruction_descriptor(BN, PAIR ? 2 * kBM : kBM);
+            constexpr uint32_t idesc = instruction_descriptor(BN);
             const int me = warp - 1;
             // stages a tile takes up: its blocks, and with a fixed issuer per stage one that is passed over when their number is odd
             const int stride = S::kStagePerIssuer ? kblocks + (kblocks & 1) : kblocks;
@@ -397,16 +399,16 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                         for (int j = 0; j < kStageK / kMmaK; ++j) {
                             const uint32_t accumulate = j == 0 ? 0u : 1u;  // every block starts a fresh sum
                             const uint64_t step = uint64_t(j * kMmaK >> 4);
-                            issue_mma(d, a_desc + step, b_desc + step, idesc, accumulate);
-                            if (S::kHilo) issue_mma(d + BN, a_lo_desc + step, b_desc + step, idesc, accumulate);
+                            mma_i8(d, a_desc + step, b_desc + step, idesc, accumulate);
+                            if (S::kHilo) mma_i8(d + BN, a_lo_desc + step, b_desc + step, idesc, accumulate);
                         }
-                        commit(bar_empty + 8 * stage);
-                        commit(bar_acc_full + 8 * acc);
+                        tc_commit(bar_empty + 8 * stage);
+                        tc_commit(bar_acc_full + 8 * acc);
                     }
                     stage += 2;  // at most one wrap per step (kStages >= 2)
                     if (stage >= kStages) { stage -= kStages; phase ^= 1u; }
                 }
-                // from block kb (the first of this thread's past the tile) to its first block of the next tile: -1, 0 or 1 stages
+                // from block kb (the first of this warp's past the tile) to its first block of the next tile: -1 to 2 stages, one wrap at most
                 const int move = stride + me - kb;
                 stage += move;
                 if (stage >= kStages) { stage -= kStages; phase ^= 1u; }
@@ -739,7 +741,7 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                         // every column of this warp's part of the buffer is in registers: the buffer goes back to the MMAs
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) give_back(bar_acc_empty + 8 * BUFFER);
+                        if (lane == 0) mbar_arrive(bar_acc_empty + 8 * BUFFER);
                     };
                     auto fold = [&](int chunk) {
                         const int* h = hi[chunk & 1];
@@ -1152,9 +1154,9 @@ static bool row_in_pairs(const GemmArgs& g) {
 }
 
 // Variant numbers keep the reference's meaning of the MODE (row 0 / 2 / 6, exact 1 / 7, block 10 / 11, block+g 12 / 13, exact+g 14); 0, 1 and 14
-// choose the tile shape by the rules above, 15 and 13 between 128 and 64 channels.  The others are this library's own shapes: 2 / 6 and 7 always 256 output channels per tile, 30
-// pairs of CTAs, 35 / 36 and 37 / 38 tiles of 128 / 64 channels; per-block modes: 256 channels (10, 12), 128 (16), 64 (17, 18), exact+g 128
-// (24) and 64 (19); 20 is 10 with eight drain warps of 128 columns instead of sixteen of 64 (fewer instructions per output, fewer
+// choose the tile shape by the rules above, 15 and 13 between 128 and 64 channels.  The others are this library's own shapes: 2 / 6 and 7
+// always 256 output channels per tile, 30 pairs of CTAs, 35 / 36 and 37 / 38 tiles of 128 / 64 channels; per-block modes: 256 channels
+// (10, 12), 128 (16), 64 (17, 18), exact+g 128 (24) and 64 (19); 20 is 10 with eight drain warps of 128 columns instead of sixteen of 64 (fewer instructions per output, fewer
 // warps to hide latencies with), 22 another name of 12.
 template <class T> static int dispatch(const GemmArgs& g, int variant, cudaStream_t stream) {
     const bool copies = g.ys && g.count > 1;  // several destinations: the wide staging tiles, single CTAs, 256 columns (exact+g: 128)

@@ -16,7 +16,7 @@ WQ_DEVICE uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta
 // that issues TMA or tensor-core instructions runs its loop with the whole warp and only the issue under elect_one(): its loop variables and
 // descriptors then live in uniform registers, from which these instructions take their operands.  In a loop that lane 0 runs alone every
 // operand is moved there first, at each instruction, on issue slots that the drain warps want.  Measured, loops of lane 0 -> this form (GEMM alone):
-// exact+g 32768 x 5120 x 5120 2007 -> 1678 us, block+g 1446 -> 1312 (pairs), block 1393 -> 1126 (128-channel tiles), row 557 -> 550.
+// exact+g 32768 x 5120 x 5120 2007 -> 1678 us, block 1393 -> 1126 (128-channel tiles), row 557 -> 550.
 WQ_DEVICE int uniform_warp() { return __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0); }
 WQ_DEVICE bool elect_one() {
     uint32_t elected;
