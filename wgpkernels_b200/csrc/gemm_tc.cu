@@ -1120,12 +1120,15 @@ template <class T, int MODE, int BN, int PARTS = 4> static int launch_width(cons
 }
 
 // ---- tile shapes ----------------------------------------------------------------------------------------------------
-// Tile width where it is chosen here (row, exact, exact+g, and the narrow tiles of block and block+g): the fewest rounds of tiles over the SMs, weighted with what one block
-// of K costs a tile.  row and exact are bound by bringing operands into the SM (64 bytes a clock), so a block costs the bytes of A (the rows
-// that exist) and B; the per-block modes by the conversions of their drain, so by the columns and a constant share (waits, hand-overs).  Wide tiles win
-// whenever there are several rounds of them; a few row tiles alone leave most SMs idle with 256 columns.  Measured (quantizer and GEMM, 256
-// columns always -> this rule): exact 64 x 5120 x 5120 29.7 -> 21.4 us, 128 x 5120 x 15360 32.4 -> 23.7, 200 x 4096 x 4096 26.0 -> 19.3; exact+g (128
-// columns before) 100 x 4096 x 4096 30.2 -> 21.8; block (128 before) 64 x 5120 x 5120 21.4 -> 15.8, 128 x 4096 x 14336 stays with 128 (20.1; 64: 23.5); row 64 x 5120 x 5120 18.5 -> 16.7; 1560 x 5120 x 5120 stays with 256 (62.3).
+// Tile width where it is chosen here (row, exact, exact+g, and the narrow tiles of block and block+g): the fewest rounds of tiles over the SMs,
+// weighted with what one block of K costs a tile.  row and exact are bound by bringing operands into the SM (64 bytes a clock), so a block
+// costs the bytes of A (the rows that exist) and B; the per-block modes by the conversions of their drain, so by the columns and a constant
+// share (waits, hand-overs).  Wide tiles win whenever there are several rounds of them; a few row tiles alone leave most SMs idle with 256
+// columns.  Measured (quantizer and GEMM, 256 columns always -> this rule): exact 64 x 5120 x 5120 29.7 -> 21.4 us, 128 x 5120 x 15360
+// 32.4 -> 23.7, 200 x 4096 x 4096 26.0 -> 19.3; exact+g (128 columns before) 100 x 4096 x 4096 30.2 -> 21.8; block (128 before)
+// 64 x 5120 x 5120 21.4 -> 15.8; row 64 x 5120 x 5120 18.5 -> 16.7.  Against every width of the mode over 30 sizes of 33 to 8192 tokens (GEMM
+// alone) the choice is within 3 % of the best, with these exceptions: 187 x 11096 x 3584 (three rounds of 64 columns chosen over two of
+// 128: exact+g 41.9 us, 36.6 with 128; block 25.2, 22.6) and 34 x 7368 x 2432 (row 9.8, 8.8 with 128).
 static int tile_columns(const GemmArgs& g, bool hilo, bool per_block) {
     const int64_t sms = g.sms > 0 ? g.sms : 148, row_tiles = (g.m + kBM - 1) / kBM;
     const int64_t a_bytes = int64_t(g.m < kBM ? g.m : kBM) * kStageK * (hilo ? 2 : 1);
@@ -1144,7 +1147,9 @@ static int tile_columns(const GemmArgs& g, bool hilo, bool per_block) {
 
 // `row` on CTA pairs: a pair brings B in once for 256 rows (32 instead of 48 KiB per SM and block of K), so the operand feed no longer
 // holds the MMAs back.  Measured on 32768 x 5120 x 5120: 521 us against 570 (3290 and 3020 TOPS, at the power limit from there on:
-// 4170 with zeros for operands).  `exact` is at that limit with single CTAs already (9007 x 15360 x 5120: 857 us, in pairs 903).  Not where the coarser tiles of 256 rows take more than that in an additional, emptier round.
+// 4170 with zeros for operands).  `exact` is at that limit with single CTAs already (9007 x 15360 x 5120: 857 us, in pairs 903).  A round
+// of pairs takes 0.92 of a round of single CTAs, so pairs are taken where the coarser tiles of 256 rows cost less than 1 / 0.92 times as
+// many rounds.  That holds for long inputs; of the 30 sizes above the worst is 187 x 11096 x 3584 (14.1 us, 13.2 on single CTAs).
 static bool row_in_pairs(const GemmArgs& g) {
     if (g.window.counter || g.m <= kBM) return false;
     const int64_t sms = g.sms > 0 ? g.sms : 148, column_tiles = int64_t((g.n + 255) / 256) * g.segments;
