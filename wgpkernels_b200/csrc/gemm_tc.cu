@@ -598,7 +598,9 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                     for (int j = 0; j < 16; ++j) {
                         const int cj = col + part16 + j;
                         if (row_ok && cj < p.n) {
-                            const float col_scale = S::kWGroup ? 1.f : sb[cj];
+                            // (through L2, as coherent as an ordinary load: the compiler then keeps the block loop of `block` on sixteen warps 1.5 %
+                            // faster, 16384 x 5120 x 13824 1152 -> 1138 us, and with eight warps 4 % slower)
+                            const float col_scale = S::kWGroup ? 1.f : PARTS == 4 ? __ldcg(sb + cj) : sb[cj];
                             float value = fmaf(mine[j] * row_scale, col_scale, bias ? as_float(bias[cj]) : 0.f);
                             if (res) {
                                 const T* rs = rscale && p.window.span ? rscale + (out_shift + row) / p.window.span * p.window.scale_step : rscale;
