@@ -51,3 +51,10 @@ def test_warps_that_meet_at_a_named_barrier_agree_there():
     text = code("stream_tc.cu")
     assert text.index("drains_agree(ok)") < text.index('"bar.sync 1, 128;"')
     assert "drains_agree(false)" in text
+
+
+def test_a_pair_waits_for_the_commits_that_arrive_in_both_ctas():
+    """A commit of the leader's MMAs arrives on the peer's barriers as well; the peer's shared memory has to be there still."""
+    text = code("gemm_tc.cu")
+    tail = text[text.index("S::kStagePerIssuer && (kblocks & 1)"):text.index("MMA issuer" if "MMA issuer" in text else "else if (warp == 1)")]
+    assert re.search(r"if constexpr \(PAIR\) \{\s*for \(int s = 0; s < kStages && ok; \+\+s\)\s*ok = whole_warp\(wait_on\(bar_empty", tail)

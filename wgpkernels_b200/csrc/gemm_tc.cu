@@ -311,6 +311,11 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                 }
                 if (S::kStagePerIssuer && (kblocks & 1) && ++stage == kStages) stage = 0;  // the next tile starts on the first issuer's stages again
             }
+            if constexpr (PAIR) {
+                // the leader's commits arrive on the barriers of both CTAs: neither leaves before the last of them has come
+                for (int s = 0; s < kStages && ok; ++s)
+                    ok = whole_warp(wait_on(bar_empty + 8 * s, ((phases >> s) & 1u) ^ 1u, abort_flag, kTimeoutEmpty));
+            }
             if (!ok) {
                 // A pair's bytes are counted on the leader's barriers: the leader waits for both CTAs' copies, the other CTA for the leader (at
                 // the cluster barrier below).  A fill that only one of them has issued never completes its phase: time to land instead.
