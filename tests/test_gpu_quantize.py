@@ -39,6 +39,27 @@ def test_quantize_blocks_matches_reference_library(wq, shape, act, dtype):
     assert torch.equal(s, s_ref)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("shape", [(3, 128), (5, 1024 - 128), (37, 1024), (3, 1024 + 128), (300, 13824), (2, 16384 + 512)], ids=lambda s: f"{s[0]}x{s[1]}")
+def test_gelu_codes_are_the_accurate_ones(wq, shape, dtype):
+    """The block quantizer puts few elements through the accurate gelu; the row quantizer puts all of them.  On rows of one block both have the same
+    scale to find, so codes and scales are the same bits: ordinary blocks, blocks without a value above 0.35, zeros, tiny and huge values,
+    values next to nothing but one, infinities and NaN."""
+    m, k = shape
+    x = randn((m, k), torch.float32, 31)
+    for i, change in enumerate((lambda v: v * 0.05, lambda v: -v.abs() - 0.4, lambda v: v * 0, lambda v: v * 1e-6, lambda v: v * 1e4,
+                                lambda v: torch.where(v > 2.0, v, v * 1e-3))):
+        x[i::7] = change(x[i::7])
+    x = x.to(dtype)
+    x.view(-1)[5::1009] = float("inf")
+    x.view(-1)[7::1013] = -float("inf")
+    x.view(-1)[9::997] = float("nan")
+    q, s = wq.quantize_blocks(x.cuda(), 0, "gelu")
+    rows = torch.nn.functional.pad(x, (0, -k % 128)).view(-1, 128).cuda()
+    q_rows, _, s_rows = wq.quantize(rows, 0, False, "gelu")
+    assert torch.equal(q, q_rows.view(m, -1)[:, :k]) and torch.equal(s, s_rows.view(m, -1))
+
+
 @pytest.mark.parametrize("group", [16, 64, 256])
 @pytest.mark.parametrize("act", [None, "rms_norm", "gelu"])
 def test_quantize_blocks_rotated_matches_reference_library(wq, group, act):

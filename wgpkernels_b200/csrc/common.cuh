@@ -50,6 +50,15 @@ template <> WQ_DEVICE void unpack_pair<__half>(uint32_t raw, float& lo, float& h
     hi = f.y;
 }
 
+// Largest and smallest of eight 16-bit values (those that are numbers).
+template <class T> WQ_DEVICE void extremes(const uint4& raw, float& largest, float& smallest) {
+    using Pair = typename std::conditional<std::is_same<T, bf16>::value, __nv_bfloat162, __half2>::type;
+    const Pair* p = reinterpret_cast<const Pair*>(&raw);
+    const Pair high = __hmax2(__hmax2(p[0], p[1]), __hmax2(p[2], p[3])), low = __hmin2(__hmin2(p[0], p[1]), __hmin2(p[2], p[3]));
+    largest = fmaxf(float(high.x), float(high.y));
+    smallest = fminf(float(low.x), float(low.y));
+}
+
 // Eight consecutive elements at p (16-byte aligned for 16-bit types, 32 bytes for float) as floats; zeros when !valid.
 template <class T> WQ_DEVICE void load_eight(const T* p, float* v, bool valid) {
     if constexpr (sizeof(T) == 2) {
