@@ -88,6 +88,37 @@ def test_quantize_blocks_matches_oracle(wq, shape, act):
         assert np.allclose(s.cpu().numpy(), s_cpu, rtol=2e-6, atol=0)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])
+@pytest.mark.parametrize("group", [16, 64, 256])
+@pytest.mark.parametrize("k", [256, 256 * 3 + 64, 4096, 4096 + 256, 8192 + 512, 16384, 16384 + 256])
+def test_rotated_codes_match_oracle(wq, k, group, dtype):
+    """IEEE operations only, in the oracle's order: the same bits.  Rows in both layouts (up to 16384 values and beyond), last chunks that are not
+    whole, zeros, and (BF16, FP32) values whose doubles are infinite."""
+    k = k // group * group
+    x = randn((6, k), torch.float32, 33)
+    x[1], x[2, ::7] = 0, x[2, ::7] * 40
+    x[3] *= 1e-7
+    if dtype != torch.float16:
+        x[4, 3] = 2.5e38
+    x = x.to(dtype)
+    with np.errstate(over="ignore", invalid="ignore"):
+        q_cpu, s_cpu = oracle.quantize_blocks(x, group)
+        hi_cpu, lo_cpu, rs_cpu = oracle.quantize_rows(x, group, True)
+    ordinary = np.isfinite(rs_cpu)  # (the oracle leaves NaN where infinities meet)
+    q, s = wq.quantize_blocks(x.cuda(), group)
+    hi, lo, rs = wq.quantize(x.cuda(), group, True)
+    only_hi, _, only_rs = wq.quantize(x.cuda(), group, False)
+    assert ordinary.sum() == (6 if dtype == torch.float16 else 5)
+    for got, expected in ((q, q_cpu), (s, s_cpu), (hi, hi_cpu), (lo, lo_cpu), (rs, rs_cpu), (only_hi, hi_cpu), (only_rs, rs_cpu)):
+        assert np.array_equal(got.cpu().numpy()[ordinary], expected[ordinary])
+    assert torch.equal(hi, only_hi) and torch.equal(rs, only_rs)
+    # codes of rows that start on an 8-byte boundary only (what the entry points ask for)
+    spare = torch.empty(6 * k + 8, dtype=torch.int8, device="cuda")[8:].view(6, k)
+    assert wq._require().wq8_quantize(x.cuda().data_ptr(), spare.data_ptr(), None, torch.empty_like(rs).data_ptr(), 6, k, k, wq._DTYPES[dtype], group, 0, None,
+                                      0.0, wq._stream(q.device)) == 0
+    assert torch.equal(spare, hi)
+
+
 @pytest.mark.parametrize("hilo", [False, True])
 @pytest.mark.parametrize("act", ACTS)
 @pytest.mark.parametrize("shape", [(1, 8), (7, 264), (5, 5120), (3, 13824), (2, 16384 + 512)], ids=lambda s: f"{s[0]}x{s[1]}")

@@ -349,6 +349,221 @@ __global__ void __launch_bounds__(kRowThreads, CPW > 0 && CPW <= 4 ? 5 : 1) quan
     }
 }
 
+// ---- rotated rows, sixteen values a lane ---------------------------------------------------------------------------------------
+// A half warp holds a chunk of 256 as sixteen consecutive values a lane: the two low base-4 digits of the index lie inside a lane.  One exchange
+// through shared memory turns the chunk over, lane i then holds the elements i + 16 j, and the two high digits lie inside a lane as well.
+// (rotate_chunk moves the digits between lanes with 60 shuffles for eight values, one a clock and SM; this takes 20 shared-memory
+// instructions for sixteen.)  The additions are those of rotate_chunk, operand by operand, so the codes are the same.
+// Measured (4096 x 3072, FP16, groups of 256): 20.9 us with the shuffles, 12.7 so; 16384 x 3072: 77 and 47.
+constexpr int kTurnStride = 20, kTurnFloats = 16 * kTurnStride + 16;  // rows 80 bytes apart, the halves of a warp 16 banks apart: no conflicts
+
+// one digit of sixteen values whose mirrored partners are STEP apart: out[d] = (in0 + in1) + (in2 + in3) - 2 in[3 - d].  HUGE_VALUES: with
+// 2 in[3 - d] rounded first, which makes infinities of what is beyond 2^127, as rotate_chunk does.
+template <int STEP, bool HUGE_VALUES> WQ_DEVICE void h4_digit_of_sixteen(float2* v) {
+    const float2 minus_two = make_float2(-2.f, -2.f);
+    auto less_twice = [&](float2 s, float2 x) {
+        if constexpr (HUGE_VALUES) return make_float2(__fadd_rn(s.x, -__fmul_rn(2.f, x.x)), __fadd_rn(s.y, -__fmul_rn(2.f, x.y)));
+        return __ffma2_rn(x, minus_two, s);
+    };
+    if constexpr (STEP == 1) {
+#pragma unroll
+        for (int g = 0; g < 8; g += 2) {
+            const float2 a = v[g], b = v[g + 1];
+            const float sum = (a.x + a.y) + (b.x + b.y);
+            const float2 s = make_float2(sum, sum);
+            v[g] = less_twice(s, make_float2(b.y, b.x));
+            v[g + 1] = less_twice(s, make_float2(a.y, a.x));
+        }
+    } else {
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            const float2 x0 = v[g], x1 = v[g + 2], x2 = v[g + 4], x3 = v[g + 6];
+            const float2 s = __fadd2_rn(__fadd2_rn(x0, x1), __fadd2_rn(x2, x3));
+            v[g] = less_twice(s, x3);
+            v[g + 2] = less_twice(s, x2);
+            v[g + 4] = less_twice(s, x1);
+            v[g + 6] = less_twice(s, x0);
+        }
+    }
+}
+// v: elements 16 i .. + 15 of the chunk -> for groups of 64 and 256 elements i + 16 j, rotated (`turn`: this half warp's kTurnFloats)
+template <int GROUP, bool HUGE_VALUES> WQ_DEVICE void rotate_sixteen(float2* v, float* turn, int i) {
+    h4_digit_of_sixteen<1, HUGE_VALUES>(v);
+    h4_digit_of_sixteen<4, HUGE_VALUES>(v);
+    if constexpr (GROUP > 16) {
+        __syncwarp();  // the chunk before this one has been read
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) *reinterpret_cast<float4*>(turn + i * kTurnStride + 2 * j) = make_float4(v[j].x, v[j].y, v[j + 1].x, v[j + 1].y);
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = make_float2(turn[2 * j * kTurnStride + i], turn[(2 * j + 1) * kTurnStride + i]);
+        h4_digit_of_sixteen<1, HUGE_VALUES>(v);
+        if constexpr (GROUP == 256) h4_digit_of_sixteen<4, HUGE_VALUES>(v);
+    }
+}
+// The rotation keeps the values' root mean square (but for its factor): where no output is as large as this, nothing on the way was.
+constexpr float kHuge = 1e38f;
+// Sixteen codes, the low bytes of c in the order rotate_sixteen leaves the values in -> the bytes 16 i .. + 15 of the chunk, stored (rows of codes
+// need 8-byte alignment only).
+template <int GROUP> WQ_DEVICE void store_sixteen(const uint32_t* c, float* turn, int i, int8_t* at, bool valid) {
+    uint4 word;
+    if constexpr (GROUP == 16) {
+        word = make_uint4(low_bytes(c[0], c[1], c[2], c[3]), low_bytes(c[4], c[5], c[6], c[7]), low_bytes(c[8], c[9], c[10], c[11]),
+                          low_bytes(c[12], c[13], c[14], c[15]));
+    } else {
+        uint8_t* bytes = reinterpret_cast<uint8_t*>(turn);
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) bytes[16 * j + i] = uint8_t(c[j]);
+        __syncwarp();
+        word = *reinterpret_cast<const uint4*>(bytes + 16 * i);
+    }
+    if (!valid) return;
+    if ((reinterpret_cast<uintptr_t>(at) & 15) == 0) {
+        *reinterpret_cast<uint4*>(at) = word;
+    } else {
+        *reinterpret_cast<uint2*>(at) = make_uint2(word.x, word.y);
+        *reinterpret_cast<uint2*>(at + 8) = make_uint2(word.z, word.w);
+    }
+}
+template <class T> WQ_DEVICE void load_sixteen(const T* p, float2* v, bool valid) {
+    float low[8], high[8];
+    load_eight(p, low, valid);
+    load_eight(p + 8, high, valid);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        v[j] = make_float2(low[2 * j], low[2 * j + 1]);
+        v[j + 4] = make_float2(high[2 * j], high[2 * j + 1]);
+    }
+}
+// Codes of t = v inv.  PLAIN: every t is a number within 127.5 of zero, so one addition rounds it; else by the conversion, which saturates and
+// makes 0 of what is no number.  (Scalar products: the compiler fuses a two-wide one with the addition behind it, __fmul2_rn() and
+// mul.rn.f32x2 alike, which puts values next to a tie on the wrong side.)
+template <bool PLAIN> WQ_DEVICE void codes_of_sixteen(const float2* v, const float2* inv, uint32_t* codes) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        const float t = __fmul_rn(j & 1 ? v[j / 2].y : v[j / 2].x, inv[j >> 3].x);
+        if constexpr (PLAIN) codes[j] = __float_as_uint(__fadd_rn(t, kRoundMagic));
+        else codes[j] = uint32_t(max(-128, min(127, __float2int_rn(t))));
+    }
+}
+
+template <class T, int GROUP>
+__global__ void __launch_bounds__(256) quantize_blocks_rotated(const T* __restrict__ x, int8_t* __restrict__ q, float* __restrict__ scale, int64_t row0, int k,
+                                                               int64_t ldx, RowShift shift) {
+    __shared__ __align__(16) float turns[16 * kTurnFloats];
+    dependents_may_start();
+    const int i = threadIdx.x & 15, half = threadIdx.x >> 4;
+    const int base = (blockIdx.x * 16 + half) * kChunk;
+    if (base - (half & 1) * kChunk >= k) return;  // both halves of a warp, or none
+    float* turn = turns + half * kTurnFloats;
+    const int kblocks = (k + kBlockK - 1) / kBlockK;
+    const int64_t row = row0 + blockIdx.y;
+    const int col = base + 16 * i;
+    float2 v[8];
+    const T* src = first_row(x, ldx, shift) + row * ldx + col;
+    load_sixteen(src, v, col < k);
+    rotate_sixteen<GROUP, false>(v, turn, i);
+    float strict = 0.f;  // absmax, or NaN
+#pragma unroll
+    for (int j = 0; j < 8; ++j) strict = magnitude_or_nan(strict, magnitude_or_nan(v[j].x, v[j].y));
+    const bool ordinary = __all_sync(0xffffffffu, fabsf(strict) < kHuge);
+    if (!std::is_same<T, __half>::value && !ordinary) {
+        load_sixteen(src, v, col < k);
+        rotate_sixteen<GROUP, true>(v, turn, i);
+    }
+    // absmax of the chunk's two blocks: lanes 0-7 end with the first block's, lanes 8-15 with the second's.  (In groups of 16 a lane's values
+    // lie in one block, else eight in each.)
+    float part[2] = {0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) part[j >> 2] = fmaxf(part[j >> 2], fmaxf(fabsf(v[j].x), fabsf(v[j].y)));
+    float amax = fmaxf(part[0], part[1]);
+    if constexpr (GROUP > 16) amax = fmaxf(i & 8 ? part[1] : part[0], __shfl_xor_sync(0xffffffffu, i & 8 ? part[0] : part[1], 8));
+#pragma unroll
+    for (int d = 4; d > 0; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
+    const int block = base / kBlockK + (i >> 3);
+    const float own_inv = amax > 0.f ? 127.f / amax : 0.f;
+    if ((i & 7) == 0 && block < kblocks) scale[row * kblocks + block] = amax * group_norm<GROUP>() / 127.f;
+    float2 inv[2] = {make_float2(own_inv, own_inv), make_float2(own_inv, own_inv)};
+    if constexpr (GROUP > 16) {
+        const float other = __shfl_xor_sync(0xffffffffu, own_inv, 8);
+        inv[i & 8 ? 0 : 1] = make_float2(other, other);
+    }
+    uint32_t c[16];
+    if (ordinary && __all_sync(0xffffffffu, own_inv < kHuge)) codes_of_sixteen<true>(v, inv, c);
+    else codes_of_sixteen<false>(v, inv, c);
+    store_sixteen<GROUP>(c, turn, i, q + row * k + col, col < k);
+}
+
+// One scale per row: a CTA per row, CPH chunks a half warp (K <= 4096 CPH), as many warps as the row has work for.
+template <class T, int GROUP, bool HILO, int CPH>
+__global__ void __launch_bounds__(256) quantize_rows_rotated(const T* __restrict__ x, int8_t* __restrict__ hi, int8_t* __restrict__ lo, float* __restrict__ scale,
+                                                             int k, int64_t ldx, RowShift shift) {
+    __shared__ __align__(16) float turns[16 * kTurnFloats];
+    __shared__ float max_slots[8];
+    dependents_may_start();
+    const int i = threadIdx.x & 15, half = threadIdx.x >> 4, halves = blockDim.x >> 4;
+    float* turn = turns + half * kTurnFloats;
+    const int64_t row = blockIdx.x;
+    const T* src = first_row(x, ldx, shift) + row * ldx;
+    float2 v[CPH][8];
+#pragma unroll
+    for (int n = 0; n < CPH; ++n) {
+        const int col = (half + n * halves) * kChunk + 16 * i;
+        load_sixteen(src + col, v[n], col < k);
+    }
+    float strict = 0.f;  // absmax, or NaN
+#pragma unroll
+    for (int n = 0; n < CPH; ++n) {
+        rotate_sixteen<GROUP, false>(v[n], turn, i);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) strict = magnitude_or_nan(strict, magnitude_or_nan(v[n][j].x, v[n][j].y));
+    }
+    float amax = fabsf(strict);
+    const bool ordinary = __all_sync(0xffffffffu, amax < kHuge);
+    if (!ordinary) {
+        amax = 0.f;
+#pragma unroll
+        for (int n = 0; n < CPH; ++n) {
+            if constexpr (!std::is_same<T, __half>::value) {
+                const int col = (half + n * halves) * kChunk + 16 * i;
+                load_sixteen(src + col, v[n], col < k);
+                rotate_sixteen<GROUP, true>(v[n], turn, i);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fmaxf(fabsf(v[n][j].x), fabsf(v[n][j].y)));
+        }
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
+    if ((threadIdx.x & 31) == 0) max_slots[threadIdx.x >> 5] = amax;
+    __syncthreads();
+    for (int w = 0; w < int(blockDim.x >> 5); ++w) amax = fmaxf(amax, max_slots[w]);
+    const float row_inv = amax > 0.f ? 127.f / amax : 0.f;
+    if (threadIdx.x == 0) scale[row] = amax * group_norm<GROUP>() / 127.f;
+    const float2 inv[2] = {make_float2(row_inv, row_inv), make_float2(row_inv, row_inv)};
+    const bool plain = ordinary && row_inv < kHuge;  // (the same in all lanes of a warp)
+#pragma unroll
+    for (int n = 0; n < CPH; ++n) {
+        const int col = (half + n * halves) * kChunk + 16 * i;
+        uint32_t h[16], l[16];
+        if constexpr (HILO) {  // as store_row_codes
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const float t = (j & 1 ? v[n][j / 2].y : v[n][j / 2].x) * row_inv;
+                const int code = __float2int_rn(t);
+                h[j] = uint32_t(max(-128, min(127, code)));
+                l[j] = uint32_t(max(-128, min(127, __float2int_rn((t - float(code)) * 254.f))));
+            }
+        } else {
+            if (plain) codes_of_sixteen<true>(v[n], inv, h);
+            else codes_of_sixteen<false>(v[n], inv, h);
+        }
+        store_sixteen<GROUP>(h, turn, i, hi + row * k + col, col < k);
+        if constexpr (HILO) store_sixteen<GROUP>(l, turn, i, lo + row * k + col, col < k);
+    }
+}
+
 // ---- few-token paths: op(x), rotated, rounded once to T ---------------------------------------------------------------
 template <class T, int GROUP, int ACT>
 __global__ void __launch_bounds__(kRowThreads) transform_rows(const T* __restrict__ x, T* __restrict__ out, int k, int64_t ldx,
@@ -438,7 +653,8 @@ static int launch_blocks(const void* x, int8_t* q, float* scale, int m, int k, i
         const int chunks = (k + kChunk - 1) / kChunk, per_cta = 8 * (kGelu ? kGeluChunks : 1);
         for (int64_t row0 = 0; row0 < m; row0 += 65535) {
             const dim3 grid((chunks + per_cta - 1) / per_cta, unsigned(m - row0 < 65535 ? m - row0 : 65535));
-            if constexpr (kGelu) quantize_blocks_gelu<T><<<grid, 256, 0, stream>>>(src, q, scale, row0, k, ldx, shift);
+            if constexpr (GROUP > 0 && ACT == kActNone) quantize_blocks_rotated<T, GROUP><<<dim3((chunks + 15) / 16, grid.y), 256, 0, stream>>>(src, q, scale, row0, k, ldx, shift);
+            else if constexpr (kGelu) quantize_blocks_gelu<T><<<grid, 256, 0, stream>>>(src, q, scale, row0, k, ldx, shift);
             else quantize_blocks_items<T, GROUP, ACT><<<grid, 256, 0, stream>>>(src, q, scale, row0, k, ldx, shift);
         }
     }
@@ -474,6 +690,18 @@ static int launch_rows(const void* x, int8_t* hi, int8_t* lo, float* scale, int 
                        const RowShift& shift, cudaStream_t stream) {
     auto src = static_cast<const T*>(x);
     auto aw = static_cast<const T*>(act_weight);
+    // (rms_norm: the order of the row's sum is that of eight values a lane; gelu and swiglu: how their last product and the rotation's first sum
+    // are fused is that kernel's)
+    if constexpr (GROUP > 0 && ACT == kActNone) {
+        if (k <= 16384) {
+            const int chunks = (k + kChunk - 1) / kChunk, per_half = k <= 4096 ? 1 : k <= 8192 ? 2 : 4;
+            const int threads = 32 * ((chunks + 2 * per_half - 1) / (2 * per_half));
+            if (per_half == 1) quantize_rows_rotated<T, GROUP, HILO, 1><<<m, threads, 0, stream>>>(src, hi, lo, scale, k, ldx, shift);
+            else if (per_half == 2) quantize_rows_rotated<T, GROUP, HILO, 2><<<m, threads, 0, stream>>>(src, hi, lo, scale, k, ldx, shift);
+            else quantize_rows_rotated<T, GROUP, HILO, 4><<<m, threads, 0, stream>>>(src, hi, lo, scale, k, ldx, shift);
+            return int(cudaGetLastError());
+        }
+    }
     if (k <= 2048) quantize_rows<T, GROUP, HILO, ACT, 1><<<m, kRowThreads, 0, stream>>>(src, hi, lo, scale, k, ldx, aw, eps, shift);
     else if (k <= 4096) quantize_rows<T, GROUP, HILO, ACT, 2><<<m, kRowThreads, 0, stream>>>(src, hi, lo, scale, k, ldx, aw, eps, shift);
     else if (k <= 8192) quantize_rows<T, GROUP, HILO, ACT, 4><<<m, kRowThreads, 0, stream>>>(src, hi, lo, scale, k, ldx, aw, eps, shift);
