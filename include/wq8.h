@@ -163,6 +163,15 @@ int64_t wq8_stream_planes_workspace(int m, int n, int k, int sms);
 int wq8_stream_planes(const void* x, int64_t ldx, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale,
                       void* y, int m, int n, int k, int dtype, int sms, void* workspace, wq8_stream_t stream);
 
+/* The same linear for one to four tokens with its input operation (act: 0 none, 2 swiglu -- rows of 2 K, gate | value --, 3 gelu) in one launch and
+ * without workspace: op(X) is rounded to X's type, as wq8_transform_rows does, and split into digit planes by every CTA for itself while its
+ * first weights are on their way.  For shapes that wq8_few_takes() (1, else 0: the shapes of wq8_stream_planes whose digits fit beside the
+ * weights; -2 otherwise); x 8-byte aligned, ldx a multiple of 4, w 16-byte aligned.  No counterpart in the reference (which launches the
+ * input operation and the product separately). */
+int wq8_few_takes(int m, int n, int k, int act, int sms);
+int wq8_few(const void* x, int64_t ldx, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale, void* y,
+            int m, int n, int k, int dtype, int act, int sms, wq8_stream_t stream);
+
 /* wq8_small for callers that cannot allocate device memory (no counterpart in the reference, which always takes caller scratch).
  * A host that reaches this library through a bare FFI with buffers it was handed, a serving loop under a fixed memory budget, code
  * running during CUDA graph capture or in a section where cudaMalloc is not allowed: none of them can supply the K-split scratch

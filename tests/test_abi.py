@@ -207,3 +207,16 @@ def test_a_library_without_this_modules_additions_is_reported(tmp_path):
     with pytest.raises(RuntimeError, match="rebuild it"):
         int8.load_library(library)
     assert int8._lib is loaded
+
+
+def test_one_launch_few_token_arguments(lib):
+    lib.wq8_few.argtypes = [p, i64, p, p, p, p, p, p, i, i, i, i, i, i, p]
+    one, odd = ctypes.c_void_p(16), ctypes.c_void_p(20)  # never dereferenced: the checks come first
+
+    def call(x=one, ldx=4096, w=one, m=1, k=4096, dtype=1, act=0):
+        return lib.wq8_few(x, ldx, w, one, None, None, None, one, m, 512, k, dtype, act, 148, None)
+
+    assert call(m=0) == 0
+    assert call(dtype=2) == -1
+    assert call(m=5) == call(k=1024) == call(k=4096 + 64) == call(act=1) == call(act=7) == -2
+    assert call(x=odd) == call(w=odd) == call(ldx=4098) == -2

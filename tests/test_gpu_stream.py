@@ -155,3 +155,38 @@ def test_weights_straight_from_the_quantizer(wq, entry, m):
     for i, y in enumerate(got):
         assert torch.equal(y, expected[i % 2])
     assert wq.debug_status() == 0
+
+
+FEW_SHAPES = [(8, 2048), (40, 2048 + 128), (1000, 4096), (16 * 148 + 24, 2048 + 384), (2304, 4096)]  # (N, K): fewer items than SMs, odd runs, partial items
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("act", [None, "swiglu", "gelu"])
+@pytest.mark.parametrize("m,shape", [(m, shape) for m in (1, 2, 3, 4) for shape in FEW_SHAPES] + [(1, (520, 16384)), (1, (264, 5120)), (2, (520, 8192))], ids=str)
+def test_input_operation_and_stream_in_one_launch(wq, m, shape, act, dtype):
+    """wq8_few: op(x) rounded as transform_rows rounds it, then the oracle's product; the residual in place; the same bits every time."""
+    n, k = shape
+    assert wq._require().wq8_few_takes(m, n, k, wq.ACTS[act], 148) == 1
+    _, w, sw, bias, res, rs = case(m, n, k, dtype, 141, True)
+    x = randn((m, 2 * k if act == "swiglu" else k), dtype, 142)
+    x[:, ::131] *= 60
+    gx, gw, gsw, gbias, gres, grs = cuda(x, w, sw, bias, res, rs)
+    prepared = wq.transform_rows(gx, 0, act).cpu() if act else x
+    target = gres.clone()
+    y = wq.linear(gx, gw, gsw, gbias, mode="lines", act=act, residual=target, residual_scale=grs, out=target)
+    assert y is target
+    assert rel(y, oracle.weight_only(prepared, w.numpy(), sw.numpy(), bias, res, rs, dtype)) < 1e-3
+    assert torch.equal(y, wq.linear(gx, gw, gsw, gbias, mode="small" if k % 64 == 0 else "lines", act=act, residual=gres, residual_scale=grs))
+    # rows of a wider matrix, and no bias or residual
+    if act != "swiglu":
+        wide = torch.zeros(m, k + 264, dtype=dtype, device="cuda")
+        wide[:, 132:132 + k] = gx
+        assert torch.equal(wq.linear(wide[:, 132:132 + k], gw, gsw, mode="lines", act=act), wq.linear(gx, gw, gsw, mode="lines", act=act))
+    assert wq.debug_status() == 0
+
+
+def test_one_launch_for_the_shapes_it_is_made_for(wq):
+    takes = wq._require().wq8_few_takes
+    assert [takes(m, 4096, 4096, 0, 148) for m in (1, 2, 3, 4, 5)] == [1, 1, 1, 1, 0]
+    assert [takes(1, 4096, k, 0, 148) for k in (1024, 2048, 2048 + 64, 16384, 16384 + 128)] == [0, 1, 0, 1, 0]
+    assert [takes(1, 4096, 4096, act, 148) for act in (0, 1, 2, 3)] == [1, 0, 1, 1]

@@ -99,6 +99,15 @@ WQ_DEVICE uint32_t pack_bytes(int a, int b, int c, int d) {
     return word;
 }
 
+// The low bytes of four words, the first one lowest.
+WQ_DEVICE uint32_t low_bytes(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    uint32_t ab, cd, word;
+    asm("prmt.b32 %0, %1, %2, 0x0040;" : "=r"(ab) : "r"(a), "r"(b));
+    asm("prmt.b32 %0, %1, %2, 0x0040;" : "=r"(cd) : "r"(c), "r"(d));
+    asm("prmt.b32 %0, %1, %2, 0x5410;" : "=r"(word) : "r"(ab), "r"(cd));
+    return word;
+}
+
 // ---- input operations, FP32 (the expression shapes fix the rounding: they are part of the numerical contract) ----
 WQ_DEVICE float gelu_tanh(float x) {
     const float inner = 0.7978845608028654f * (x + 0.044715f * (x * x * x));
@@ -257,6 +266,11 @@ inline cudaError_t launch_after_previous(void (*kernel)(Params...), dim3 grid, d
 // swizzle, zero fill outside; false when the driver entry point is missing or refuses the description.
 bool make_byte_matrix_map(CUtensorMap* map, const void* base, int rows, int row_bytes, int box_bytes, int box_rows);
 int stream_status_take();  // stream.cu: status of the weight-streaming kernels on the current device (0 = fine), cleared by the call
+// stream_few.cu: input operation, digit planes and weight stream of one to four tokens in one launch, for shapes it takes
+bool stream_few_takes(int m, int k);
+int stream_few_launch(const void* x, int64_t ldx, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale, void* y, int m,
+                      int n, int k, int dtype, int act, int sms, cudaStream_t stream);
+int stream_few_status_take();
 // stream_tc.cu: the few-token linear on tcgen05 (digit planes): scratch bytes of a shape (0: not this kernel's shape; *counter_bytes: its
 // tile counters), the launch (x already transformed; workspace and zeroed counters of those sizes), and its status word
 int64_t stream_tc_workspace(int m, int n, int k, int sms, int64_t* counter_bytes);

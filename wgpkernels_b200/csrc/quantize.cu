@@ -161,15 +161,6 @@ WQ_DEVICE float magnitude_or_nan(float a, float b) {
     asm("max.NaN.xorsign.abs.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
     return r;
 }
-// The low bytes of four words, the first one lowest.
-WQ_DEVICE uint32_t low_bytes(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    uint32_t ab, cd, word;
-    asm("prmt.b32 %0, %1, %2, 0x0040;" : "=r"(ab) : "r"(a), "r"(b));
-    asm("prmt.b32 %0, %1, %2, 0x0040;" : "=r"(cd) : "r"(c), "r"(d));
-    asm("prmt.b32 %0, %1, %2, 0x5410;" : "=r"(word) : "r"(ab), "r"(cd));
-    return word;
-}
-
 template <class T>
 __global__ void __launch_bounds__(256, 5) quantize_blocks_gelu(const T* __restrict__ x, int8_t* __restrict__ q, float* __restrict__ scale, int64_t row0, int k,
                                                             int64_t ldx, RowShift shift) {

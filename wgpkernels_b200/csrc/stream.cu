@@ -5,7 +5,8 @@
 //                  mma.sync.m16n8k16 (what wq8_gemv_lines runs, and wq8_small without scratch)
 //   stream_planes  up to 8 tokens: the activations as INT8 digit planes, the weights into mma.sync.m16n8k32.s8 untouched
 //   direct_rows    every other shape and alignment, on plain CUDA cores, with an optional split of K over CTAs
-// and stream_tc.cu holds the tcgen05 kernel that wq8_small runs with its caller's scratch (up to 32 tokens).
+// stream_few.cu holds the one that does up to 4 tokens and their input operation in one launch (what wq8_few runs, and wq8_stream_planes where the
+// digits of all of K fit beside the weights), and stream_tc.cu the tcgen05 kernel that wq8_small runs with its caller's scratch (up to 32 tokens).
 // Together they replace w8a16_small / gemv_lines of the reference (wgpkernels/int8/int8_gemm.cu:1039-1151, 1772-1810): same values up
 // to FP32 summation order.
 #include "common.cuh"
@@ -780,9 +781,9 @@ int stream_status_take() {
     const int zero = 0;
     if (cudaMemcpyFromSymbol(&code, g_stream_status, sizeof(int)) != cudaSuccess) return -1;
     if (code) cudaMemcpyToSymbol(g_stream_status, &zero, sizeof(int));
-    const int tensor_core_kernel = stream_tc_status_take();
-    if (tensor_core_kernel < 0) return -1;
-    return code ? code : tensor_core_kernel;
+    const int tensor_core_kernel = stream_tc_status_take(), one_launch = stream_few_status_take();
+    if (tensor_core_kernel < 0 || one_launch < 0) return -1;
+    return code ? code : tensor_core_kernel ? tensor_core_kernel : one_launch;
 }
 
 static int device_sms() {
@@ -816,8 +817,23 @@ WQ_API int wq8_stream_planes(const void* x, int64_t ldx, const int8_t* w, const 
         return -2;
     const int rows = plan_bulk(m, n, k, sms);
     if (!rows) return -2;
+    if (stream_few_takes(m, k)) return stream_few_launch(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, dtype, kActNone, sms, stream);
     if (dtype == 0) return launch_planes<__half>(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, rows, sms, workspace, stream);
     return launch_planes<bf16>(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, rows, sms, workspace, stream);
+}
+
+// The few-token linear with its input operation in one launch, where the digits of all of K fit beside the weight rings (stream_few.cu): the
+// shapes of wq8_stream_planes with few enough m K, without an input operation, with swiglu or with gelu.
+WQ_API int wq8_few_takes(int m, int n, int k, int act, int sms) {
+    return wq8_stream_planes_workspace(m, n, k, sms) > 0 && stream_few_takes(m, k) && (act == kActNone || act == kActSwiglu || act == kActGelu);
+}
+
+WQ_API int wq8_few(const void* x, int64_t ldx, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale, void* y, int m,
+                   int n, int k, int dtype, int act, int sms, cudaStream_t stream) {
+    if (m <= 0 || n <= 0) return 0;
+    if (dtype != 0 && dtype != 1) return -1;
+    if (!wq8_few_takes(m, n, k, act, sms) || ldx % 4 || (reinterpret_cast<uintptr_t>(x) & 7) || (reinterpret_cast<uintptr_t>(w) & 15)) return -2;
+    return stream_few_launch(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, dtype, act, sms, stream);
 }
 
 // The tensor-core kernel takes every shape with K a multiple of 128 and at most 1024 channel tiles (the counter buffer callers keep).
