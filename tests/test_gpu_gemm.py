@@ -414,3 +414,36 @@ def test_explicit_tile_shapes_match_oracle(wq, shape, mode, variant):
     y = wq.gemm(dev(a), dev(a_lo), dev(sa), dev(b), dev(sb), dev(bias), dtype, 0, variant, residual=dev(res), residual_scale=dev(rs))
     expected = oracle.gemm(base, a.numpy(), None if a_lo is None else a_lo.numpy(), sa.numpy(), b.numpy(), sb.numpy(), bias, res, rs, dtype)
     assert rel(y, expected) < 1e-3 and wq.debug_status() == 0
+
+
+@pytest.mark.parametrize("mode", ["row", "exact"])
+@pytest.mark.parametrize("m", [1, 16, 17, 29, 100, 127, 128])
+@pytest.mark.parametrize("shape", [(8, 256), (129, 384 + 16), (1000, 1040), (5120, 2064), (9472, 512)], ids=str)
+def test_k_split_over_a_cluster(wq, shape, m, mode):
+    """Up to 128 rows on clusters of CTAs: integer sums in any order are the same integers, so the outputs are the bits of the kernel that has all of
+    K in one CTA.  Odd numbers of rows and channels, partial blocks of K, strided outputs, the residual in place."""
+    n, k = shape
+    dtype = torch.bfloat16 if m % 2 else torch.float16
+    _, a, a_lo, sa, b, sb, bias, res, rs = operands(mode, m, n, k, dtype, 35, True)
+    a, a_lo, sa, b, sb, bias, res, rs = (None if t is None else t.cuda() for t in (a, a_lo, sa, b, sb, bias, res, rs))
+    one_cta, cluster = (2, 40) if mode == "row" else (7, 41)
+    call = lambda variant, **kw: wq.gemm(a, a_lo, sa, b, sb, bias, dtype, 0, variant, **kw)
+    assert torch.equal(call(cluster), call(one_cta))
+    expected = call(one_cta, residual=res, residual_scale=rs)
+    target = res.clone()
+    assert torch.equal(call(cluster, residual=target, residual_scale=rs, out=target), expected)
+    assert torch.equal(wq.gemm(a, a_lo, sa, b, sb, bias, dtype, 0, 0 if mode == "row" else 1, residual=res, residual_scale=rs), expected)
+    if n % 8 == 0:
+        wide, wide_res = torch.zeros(m, n + 24, dtype=dtype, device="cuda"), torch.zeros(m, n + 40, dtype=dtype, device="cuda")
+        wide_res[:, 16:16 + n] = res
+        call(cluster, residual=wide_res[:, 16:16 + n], residual_scale=rs, out=wide[:, 8:8 + n])
+        assert torch.equal(wide[:, 8:8 + n], expected) and not wide[:, :8].any() and not wide[:, 8 + n:].any()
+    assert wq.debug_status() == 0
+
+
+def test_k_split_is_refused_where_it_does_not_fit(wq):
+    a, b = torch.zeros(129, 512, dtype=torch.int8, device="cuda"), torch.zeros(20000, 512, dtype=torch.int8, device="cuda")
+    sa, sb = torch.ones(129, device="cuda"), torch.ones(20000, device="cuda")
+    for rows, channels, k in ((129, 256, 512), (64, 20000, 512), (64, 256, 128)):  # rows, channels for the GPU's clusters, blocks of K
+        with pytest.raises(RuntimeError, match="-2"):
+            wq.gemm(a[:rows, :k].contiguous(), None, sa[:rows], b[:channels, :k].contiguous(), sb[:channels], None, torch.bfloat16, 0, 40)

@@ -17,7 +17,7 @@ from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PACKAGE = Path(__file__).resolve().parent
-SOURCES = ("api.cu", "quantize.cu", "stream.cu", "stream_few.cu", "stream_tc.cu", "gemm_tc.cu")
+SOURCES = ("api.cu", "quantize.cu", "stream.cu", "stream_few.cu", "stream_tc.cu", "gemm_rows.cu", "gemm_tc.cu")
 PROBE_SOURCES = ("probe.cu",)
 HEADERS = ("common.cuh", "tc_ptx.cuh")
 ARCH_FLAGS = ("-gencode", "arch=compute_100a,code=sm_100a")
@@ -27,7 +27,7 @@ ARCH_FLAGS = ("-gencode", "arch=compute_100a,code=sm_100a")
 # (the copy would be taken before the load has delivered, and columns come out wrong now and then).  So these kernels do not spill at
 # all, but for one value of 'block' on 256 channels with sixteen drain warps (gemm_i8_tc<T, 2, 256, *, 0, 4, 0>): it belongs to the write-out,
 # behind the last such load -- the same kernels without their write-out spill nothing, and with half the registers for those loads as much.
-NO_SPILLS = re.compile(r"gemm_i8_tc|stream_tc|split_digits")
+NO_SPILLS = re.compile(r"gemm_i8_tc|gemm_few_rows|stream_tc|split_digits")
 SPILLS_ALLOWED = {r"gemm_i8_tcI(13__nv_bfloat16|6__half)Li2ELi256ELb[01]ELb0ELi4ELb0EE": (8, 4)}  # mangled name: bytes stored, loaded
 
 

@@ -271,6 +271,12 @@ bool stream_few_takes(int m, int k);
 int stream_few_launch(const void* x, int64_t ldx, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale, void* y, int m,
                       int n, int k, int dtype, int act, int sms, cudaStream_t stream);
 int stream_few_status_take();
+// gemm_rows.cu: `row` and `exact` of up to 128 rows, K split over the CTAs of a cluster (0 CTAs: not its shape)
+int gemm_few_rows_cluster(int m, int n, int k, int sms);
+bool gemm_few_rows_wins(int m, int n, int k, bool hilo, int sms);
+int gemm_few_rows_launch(const int8_t* a, const int8_t* a_lo, const float* sa, const int8_t* w, const float* sw, const void* bias, const void* residual,
+                         const void* rscale, void* y, int64_t ld_y, int64_t ld_residual, int m, int n, int k, bool is_bf16, int sms, cudaStream_t stream);
+int gemm_rows_status_take();
 // stream_tc.cu: the few-token linear on tcgen05 (digit planes): scratch bytes of a shape (0: not this kernel's shape; *counter_bytes: its
 // tile counters), the launch (x already transformed; workspace and zeroed counters of those sizes), and its status word
 int64_t stream_tc_workspace(int m, int n, int k, int sms, int64_t* counter_bytes);

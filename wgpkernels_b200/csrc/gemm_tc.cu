@@ -1168,16 +1168,24 @@ static bool row_in_pairs(const GemmArgs& g) {
 // Variant numbers keep the reference's meaning of the MODE (row 0 / 2 / 6, exact 1 / 7, block 10 / 11, block+g 12 / 13, exact+g 14); 0, 1 and 14
 // choose the tile shape by the rules above, 15 and 13 between 128 and 64 channels.  The others are this library's own shapes: 2 / 6 and 7
 // always 256 output channels per tile, 30 pairs of CTAs, 35 / 36 and 37 / 38 tiles of 128 / 64 channels; per-block modes: 256 channels
-// (10, 12), 128 (16), 64 (17, 18), exact+g 128 (24) and 64 (19); 20 is 10 with eight drain warps of 128 columns instead of sixteen of 64 (fewer instructions per output, fewer
+// (10, 12), 128 (16), 64 (17, 18), exact+g 128 (24) and 64 (19); 40 and 41 the kernel for up to 128 rows (gemm_rows.cu) where all its clusters
+// fit the GPU (-2 otherwise), which 0 and 1 take by its own rule; 20 is 10 with eight drain warps of 128 columns instead of sixteen of 64 (fewer instructions per output, fewer
 // warps to hide latencies with), 22 another name of 12.
 template <class T> static int dispatch(const GemmArgs& g, int variant, cudaStream_t stream) {
     const bool copies = g.ys && g.count > 1;  // several destinations: the wide staging tiles, single CTAs, 256 columns (exact+g: 128)
+    const bool plain = !copies && g.segments == 1 && !g.window.counter;
+    if (plain && (variant == 0 || variant == 1) && gemm_few_rows_wins(g.m, g.n, g.k, variant == 1, g.sms)) variant = variant == 1 ? 41 : 40;
     if (variant == 0) variant = copies ? 2 : tile_columns(g, false, false) == 256 ? (row_in_pairs(g) ? 30 : 2) : tile_columns(g, false, false) == 128 ? 35 : 36;
     if (variant == 1) variant = copies ? 7 : tile_columns(g, true, false) == 256 ? 7 : tile_columns(g, true, false) == 128 ? 37 : 38;
     const bool narrowest = !copies && tile_columns(g, false, true) == 64;
     if (variant == 14) variant = narrowest ? 19 : 24;
     if (variant == 15 && narrowest) variant = 17;
     if (variant == 13 && narrowest) variant = 18;
+    if (variant == 40 || variant == 41) {
+        if (!plain) return -3;
+        return gemm_few_rows_launch(g.a, g.a_lo, g.sa, g.b, g.sb, g.bias, g.residual, g.rscale, g.ys ? g.ys[0] : g.y, g.ld_y ? g.ld_y : g.n,
+                                    g.ld_residual ? g.ld_residual : g.n, g.m, g.n, g.k, std::is_same<T, bf16>::value, g.sms, stream);
+    }
     switch (variant) {
         case 2: case 6: return launch_width<T, kRow, 256>(g, stream);
         case 7: return launch_width<T, kExact, 256>(g, stream);
@@ -1205,8 +1213,8 @@ template <class T> static int dispatch(const GemmArgs& g, int variant, cudaStrea
 // The Mode of a variant, -1 for a number that is none.
 static int mode_of(int variant) {
     switch (variant) {
-        case 0: case 2: case 6: case 30: case 35: case 36: return kRow;
-        case 1: case 7: case 37: case 38: return kExact;
+        case 0: case 2: case 6: case 30: case 35: case 36: case 40: return kRow;
+        case 1: case 7: case 37: case 38: case 41: return kExact;
         case 10: case 11: case 15: case 16: case 17: case 20: return kBlock;
         case 12: case 13: case 18: case 22: return kBlockG;
         case 14: case 19: case 24: return kExactG;
@@ -1350,5 +1358,7 @@ WQ_API int wq8_debug_status() {
     cudaMemcpyToSymbol(g_status, &zero, sizeof(int));
     const int streaming = wq::stream_status_take();  // the weight-streaming kernels keep their own word
     if (streaming < 0) return -1;
-    return code ? code : streaming ? 100 + streaming : 0;
+    const int few_rows = wq::gemm_rows_status_take();
+    if (few_rows < 0) return -1;
+    return code ? code : few_rows ? few_rows : streaming ? 100 + streaming : 0;
 }

@@ -128,6 +128,11 @@ WQ_DEVICE uint32_t cluster_rank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
+WQ_DEVICE uint32_t cluster_size() {
+    uint32_t n;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
+    return n;
+}
 // the address of this CTA's shared-memory location `address` in CTA `rank` of the cluster
 WQ_DEVICE uint32_t in_cta(uint32_t address, uint32_t rank) {
     uint32_t mapped;
