@@ -163,14 +163,17 @@ int64_t wq8_stream_planes_workspace(int m, int n, int k, int sms);
 int wq8_stream_planes(const void* x, int64_t ldx, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale,
                       void* y, int m, int n, int k, int dtype, int sms, void* workspace, wq8_stream_t stream);
 
-/* The same linear for one to four tokens with its input operation (act: 0 none, 2 swiglu -- rows of 2 K, gate | value --, 3 gelu) in one launch and
- * without workspace: op(X) is rounded to X's type, as wq8_transform_rows does, and split into digit planes by every CTA for itself while its
- * first weights are on their way.  For shapes that wq8_few_takes() (1, else 0: the shapes of wq8_stream_planes whose digits fit beside the
- * weights; -2 otherwise); x 8-byte aligned, ldx a multiple of 4, w 16-byte aligned.  No counterpart in the reference (which launches the
- * input operation and the product separately). */
+/* The few-token linear together with its input operation (act: 0 none, 1 rms_norm with act_weight (K values of X's type, or NULL) and eps, 2 swiglu --
+ * rows of 2 K, gate | value --, 3 gelu): op(X) is rounded to X's type, as wq8_transform_rows does.  wq8_few_takes() says how a shape runs:
+ *   1  one launch, no scratch: up to four tokens, the shapes of wq8_stream_planes whose digit planes fit beside the weights, not rms_norm (every CTA
+ *      makes the planes for itself while its first weights are on their way); x 8-byte aligned, ldx a multiple of 4
+ *   2  two launches: 5 to 32 tokens, the shapes that wq8_small runs on tcgen05; slots and counters as wq8_small_workspace() reports; x and
+ *      act_weight 16-byte aligned, ldx a multiple of 8
+ *   0  not at all (-2 from wq8_few).  w 16-byte aligned.  No counterpart in the reference (which launches the input operation and the product
+ * separately). */
 int wq8_few_takes(int m, int n, int k, int act, int sms);
 int wq8_few(const void* x, int64_t ldx, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale, void* y,
-            int m, int n, int k, int dtype, int act, int sms, wq8_stream_t stream);
+            int m, int n, int k, int dtype, int act, const void* act_weight, float eps, int sms, float* slots, int* counters, wq8_stream_t stream);
 
 /* wq8_small for callers that cannot allocate device memory (no counterpart in the reference, which always takes caller scratch).
  * A host that reaches this library through a bare FFI with buffers it was handed, a serving loop under a fixed memory budget, code

@@ -209,14 +209,18 @@ def test_a_library_without_this_modules_additions_is_reported(tmp_path):
     assert int8._lib is loaded
 
 
-def test_one_launch_few_token_arguments(lib):
-    lib.wq8_few.argtypes = [p, i64, p, p, p, p, p, p, i, i, i, i, i, i, p]
-    one, odd = ctypes.c_void_p(16), ctypes.c_void_p(20)  # never dereferenced: the checks come first
+def test_few_token_arguments(lib):
+    lib.wq8_few.argtypes = [p, i64, p, p, p, p, p, p, i, i, i, i, i, p, f, i, p, p, p]
+    one, odd, scratch = ctypes.c_void_p(16), ctypes.c_void_p(20), ctypes.c_void_p(256)  # never dereferenced: the checks come first
 
-    def call(x=one, ldx=4096, w=one, m=1, k=4096, dtype=1, act=0):
-        return lib.wq8_few(x, ldx, w, one, None, None, None, one, m, 512, k, dtype, act, 148, None)
+    def call(x=one, ldx=4096, w=one, m=1, k=4096, dtype=1, act=0, slots=None, counters=None, weight=None):
+        return lib.wq8_few(x, ldx, w, one, None, None, None, one, m, 512, k, dtype, act, weight, 0.0, 148, slots, counters, None)
 
     assert call(m=0) == 0
     assert call(dtype=2) == -1
-    assert call(m=5) == call(k=1024) == call(k=4096 + 64) == call(act=1) == call(act=7) == -2
+    assert call(m=33) == call(k=1024) == call(k=4096 + 64) == call(act=1) == call(act=7) == -2
     assert call(x=odd) == call(w=odd) == call(ldx=4098) == -2
+    # more than four tokens: scratch of wq8_small, 16-byte aligned rows and norm weights
+    assert call(m=16) == call(m=16, slots=one, counters=one) == call(m=16, slots=scratch) == -2
+    assert call(m=16, slots=scratch, counters=one, x=ctypes.c_void_p(8)) == call(m=16, slots=scratch, counters=one, ldx=4100) == -2
+    assert call(m=16, slots=scratch, counters=one, act=1, weight=odd) == -2

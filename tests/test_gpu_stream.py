@@ -185,8 +185,31 @@ def test_input_operation_and_stream_in_one_launch(wq, m, shape, act, dtype):
     assert wq.debug_status() == 0
 
 
-def test_one_launch_for_the_shapes_it_is_made_for(wq):
+def test_how_the_shapes_run(wq):
     takes = wq._require().wq8_few_takes
-    assert [takes(m, 4096, 4096, 0, 148) for m in (1, 2, 3, 4, 5)] == [1, 1, 1, 1, 0]
+    assert [takes(m, 4096, 4096, 0, 148) for m in (1, 2, 3, 4, 5, 32, 33)] == [1, 1, 1, 1, 2, 2, 0]
     assert [takes(1, 4096, k, 0, 148) for k in (1024, 2048, 2048 + 64, 16384, 16384 + 128)] == [0, 1, 0, 1, 0]
-    assert [takes(1, 4096, 4096, act, 148) for act in (0, 1, 2, 3)] == [1, 0, 1, 1]
+    assert [takes(1, 4096, 4096, act, 148) for act in (0, 1, 2, 3, 4)] == [1, 0, 1, 1, 0]
+    assert [takes(9, 4096, k, act, 148) for act in (0, 1, 2, 3) for k in (128, 4096, 4096 + 64)] == [2, 2, 0] * 4
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("act", [None, "rms_norm", "swiglu", "gelu"])
+@pytest.mark.parametrize("m,n,k", [(5, 40, 128), (8, 1000, 1152), (9, 264, 4096 + 128), (16, 2048, 14336), (17, 129, 2048), (32, 520, 5120)], ids=str)
+def test_input_operation_in_the_digit_split(wq, m, n, k, act, dtype):
+    """wq8_few above four tokens: the digits of op(x) rounded as transform_rows rounds it, so the bits of wq8_small on those rows."""
+    _, w, sw, bias, res, rs = case(m, n, k, dtype, 151, True)
+    x = randn((m, 2 * k if act == "swiglu" else k), dtype, 152)
+    x[:, ::131] *= 60
+    x[1] = 0
+    norm = (1 + 0.1 * randn((k,), torch.float32, 153)).to(dtype) if act == "rms_norm" else None
+    gx, gw, gsw, gbias, gres, grs, gnorm = cuda(x, w, sw, bias, res, rs, norm)
+    prepared = wq.transform_rows(gx, 0, act, gnorm, 1e-6) if act else gx
+    expected = wq.small(prepared, gw, gsw, gbias, gres, grs)
+    target = gres.clone()
+    y = wq.linear(gx, gw, gsw, gbias, mode="small", act=act, act_weight=gnorm, eps=1e-6, residual=target, residual_scale=grs, out=target)
+    assert y is target and torch.equal(y, expected)
+    assert rel(y, oracle.weight_only(prepared.cpu(), w.numpy(), sw.numpy(), bias, res, rs, dtype)) < 1e-3
+    if act == "rms_norm":  # without a weight
+        assert torch.equal(wq.linear(gx, gw, gsw, mode="small", act=act, eps=1e-6), wq.small(wq.transform_rows(gx, 0, act, None, 1e-6), gw, gsw))
+    assert not wq._counters[0].any().item() and wq.debug_status() == 0

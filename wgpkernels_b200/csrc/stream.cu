@@ -5,7 +5,7 @@
 //                  mma.sync.m16n8k16 (what wq8_gemv_lines runs, and wq8_small without scratch)
 //   stream_planes  up to 8 tokens: the activations as INT8 digit planes, the weights into mma.sync.m16n8k32.s8 untouched
 //   direct_rows    every other shape and alignment, on plain CUDA cores, with an optional split of K over CTAs
-// stream_few.cu holds the one that does up to 4 tokens and their input operation in one launch (what wq8_few runs, and wq8_stream_planes where the
+// stream_few.cu holds the one that does up to 4 tokens and their input operation in one launch (wq8_few, and wq8_stream_planes where the
 // digits of all of K fit beside the weights), and stream_tc.cu the tcgen05 kernel that wq8_small runs with its caller's scratch (up to 32 tokens).
 // Together they replace w8a16_small / gemv_lines of the reference (wgpkernels/int8/int8_gemm.cu:1039-1151, 1772-1810): same values up
 // to FP32 summation order.
@@ -822,24 +822,31 @@ WQ_API int wq8_stream_planes(const void* x, int64_t ldx, const int8_t* w, const 
     return launch_planes<bf16>(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, rows, sms, workspace, stream);
 }
 
-// The few-token linear with its input operation in one launch, where the digits of all of K fit beside the weight rings (stream_few.cu): the
-// shapes of wq8_stream_planes with few enough m K, without an input operation, with swiglu or with gelu.
-WQ_API int wq8_few_takes(int m, int n, int k, int act, int sms) {
-    return wq8_stream_planes_workspace(m, n, k, sms) > 0 && stream_few_takes(m, k) && (act == kActNone || act == kActSwiglu || act == kActGelu);
-}
-
-WQ_API int wq8_few(const void* x, int64_t ldx, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale, void* y, int m,
-                   int n, int k, int dtype, int act, int sms, cudaStream_t stream) {
-    if (m <= 0 || n <= 0) return 0;
-    if (dtype != 0 && dtype != 1) return -1;
-    if (!wq8_few_takes(m, n, k, act, sms) || ldx % 4 || (reinterpret_cast<uintptr_t>(x) & 7) || (reinterpret_cast<uintptr_t>(w) & 15)) return -2;
-    return stream_few_launch(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, dtype, act, sms, stream);
-}
-
 // The tensor-core kernel takes every shape with K a multiple of 128 and at most 1024 channel tiles (the counter buffer callers keep).
 static int64_t tensor_core_scratch(int m, int n, int k, int sms, int64_t* counter_bytes) {
     const int64_t bytes = stream_tc_workspace(m, n, k, sms, counter_bytes);
     return bytes && *counter_bytes <= 4096 ? bytes : 0;
+}
+
+// The few-token linear with its input operation: up to four tokens in one launch where the digits of all of K fit beside the weight rings
+// (stream_few.cu; not behind rms_norm, whose row sum comes first), more in two, the input operation being part of the digit split.
+WQ_API int wq8_few_takes(int m, int n, int k, int act, int sms) {
+    if (act < kActNone || act > kActGelu) return 0;
+    if (m <= 4) return act != kActRms && wq8_stream_planes_workspace(m, n, k, sms) > 0 && stream_few_takes(m, k);
+    int64_t counter_bytes = 0;
+    return tensor_core_scratch(m, n, k, sms, &counter_bytes) ? 2 : 0;
+}
+
+WQ_API int wq8_few(const void* x, int64_t ldx, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale, void* y, int m,
+                   int n, int k, int dtype, int act, const void* act_weight, float eps, int sms, float* slots, int* counters, cudaStream_t stream) {
+    if (m <= 0 || n <= 0) return 0;
+    if (dtype != 0 && dtype != 1) return -1;
+    const int form = wq8_few_takes(m, n, k, act, sms);
+    const uintptr_t rows = reinterpret_cast<uintptr_t>(x) | uintptr_t(ldx) * 2;
+    if (!form || (reinterpret_cast<uintptr_t>(w) & 15) || (rows & (form == 1 ? 7 : 15))) return -2;
+    if (form == 1) return stream_few_launch(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, dtype, act, sms, stream);
+    if (!slots || !counters || (reinterpret_cast<uintptr_t>(slots) & 255) || (reinterpret_cast<uintptr_t>(act_weight) & 15)) return -2;
+    return stream_tc_launch(x, ldx, act, act_weight, eps, w, sw, bias, residual, rscale, y, m, n, k, dtype, sms, slots, counters, stream);
 }
 
 WQ_API void wq8_small_workspace(int m, int n, int k, int sms, int64_t* sizes) {
@@ -861,7 +868,7 @@ WQ_API int wq8_small(const void* x, int64_t ldx, const int8_t* w, const float* s
     // with the caller's scratch: the tensor-core kernel (digit planes, stream-K over all SMs)
     int64_t counter_bytes = 0;
     if (slots && counters && (reinterpret_cast<uintptr_t>(slots) & 255) == 0 && tensor_core_scratch(m, n, k, sms, &counter_bytes))
-        return stream_tc_launch(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, dtype, sms, slots, counters, stream);
+        return stream_tc_launch(x, ldx, kActNone, nullptr, 0.f, w, sw, bias, residual, rscale, y, m, n, k, dtype, sms, slots, counters, stream);
     const int rows = plan_bulk(m, n, k, sms);
     if (rows && dtype == 0) return launch_bulk<__half>(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, rows, sms, stream);
     if (rows) return launch_bulk<bf16>(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, rows, sms, stream);
@@ -966,7 +973,7 @@ WQ_API int wq8_small_static(const void* x, int64_t ldx, const int8_t* w, const f
         const cudaError_t cleared = cudaMemsetAsync(counters, 0, size_t(counter_bytes), stream);
         if (cleared != cudaSuccess) return int(cleared);
     }
-    if (tensor_core_bytes) return stream_tc_launch(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, dtype, sms, slots, counters, stream);
+    if (tensor_core_bytes) return stream_tc_launch(x, ldx, kActNone, nullptr, 0.f, w, sw, bias, residual, rscale, y, m, n, k, dtype, sms, slots, counters, stream);
     if (rows && dtype == 0) return launch_bulk<__half>(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, rows, sms, stream);
     if (rows) return launch_bulk<bf16>(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, rows, sms, stream);
     if (dtype == 0) return launch_direct<__half>(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, p, slots, counters, stream);

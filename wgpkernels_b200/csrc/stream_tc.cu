@@ -48,53 +48,92 @@ template <int TB> struct TcShape {
     static constexpr int kPieceFloats = kTcChannels * TB;            // partial sums of one piece of a tile
 };
 
-// digits: (3 TB [padded to 32 rows for TB = 8], K) int8, row p * TB + t = plane p of token slot t; scales: (K / 128, TB) float = 2^(E-7)
-// of (run, token), 0 for empty slots.  One warp per (token slot, run), 4 values per lane.
-template <class T, int TB>
-__global__ void __launch_bounds__(256) split_digits(const T* x, int64_t ldx, int8_t* __restrict__ digits, float* __restrict__ scales, int m, int k) {
+// op(x) of the tokens, rounded to T as transform_rows rounds it, and its digits: (3 TB [padded to 32 rows for TB = 8], K) int8, row p * TB + t =
+// plane p of token slot t; scales: (K / 128, TB) float = 2^(E-7) of (run, token), 0 for empty slots.  The grid is (token slots, CTAs of a row); a
+// warp takes chunks of two runs, 8 values a lane, in the order that fixes the row sum of rms_norm (one CTA a row there).
+// The input operation used to be a launch of its own (transform_rows) and the digits came from 4 values a lane with truncations in FP32: 16
+// tokens x 14336, SwiGLU, 2.3 + 2.4 us -> 2.5.
+template <class T, int TB, int ACT>
+__global__ void __launch_bounds__(kRowThreads) split_digits(const T* x, int64_t ldx, const T* act_weight, float eps, int8_t* __restrict__ digits,
+                                                            float* __restrict__ scales, int m, int k) {
+    __shared__ float slots[9];
     // This kernel may have started under the tail of the one that produced x.  Once that has finished, the stream kernel that follows may
     // start (its set-up and its first weight loads do not depend on the digits; the weights themselves may come from the kernel waited for
     // here); it waits for this grid to finish before it touches the digits.
     dependency_wait();
     dependents_may_start();
-    const int lane = threadIdx.x & 31, runs = k / kTcRun;
-    const int unit = blockIdx.x * 8 + (threadIdx.x >> 5);
-    constexpr int kRows = TcShape<TB>::kDigitRows, kSlots = kRows == 3 * TB ? TB : kRows - 2 * TB;  // TB = 8: 16 slots cover the padding rows
-    if (unit >= runs * kSlots) return;
-    const int token = unit % kSlots, run = unit / kSlots;
-    if (token >= TB) {  // padding rows of the 8-token layout (rows 24 .. 31): zeros
-        *reinterpret_cast<uint32_t*>(digits + int64_t(2 * TB + token) * k + run * kTcRun + 4 * lane) = 0u;
-        return;
-    }
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
-    if (token < m) {
-        const uint2 raw = load_8(x + int64_t(token) * ldx + run * kTcRun + 4 * lane);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, token = blockIdx.x;
+    const T* row = x + int64_t(token) * ldx;
+    const bool used = token < m;
+    auto load = [&](const T* p, float* v, bool valid) {
+        const uint4 raw = valid ? load_16(p) : make_uint4(0u, 0u, 0u, 0u);
         unpack_pair<T>(raw.x, v[0], v[1]);
         unpack_pair<T>(raw.y, v[2], v[3]);
+        unpack_pair<T>(raw.z, v[4], v[5]);
+        unpack_pair<T>(raw.w, v[6], v[7]);
+    };
+    float inv_rms = 1.f;
+    if constexpr (ACT == kActRms) {
+        float ss = 0.f;
+        for (int base = warp * kChunk; base < k; base += 8 * kChunk) {
+            float v[8];
+            load(row + base + lane * 8, v, used && base + lane * 8 < k);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) ss = fmaf(v[j], v[j], ss);
+        }
+        inv_rms = cta_inverse_rms(ss, slots, k, eps);
     }
-    float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
+    for (int base = (blockIdx.y * 8 + warp) * kChunk; base < k; base += gridDim.y * 8 * kChunk) {
+        const int col = base + lane * 8;
+        const bool valid = used && col < k;
+        float v[8];
+        load(row + col, v, valid);
+        if constexpr (ACT == kActSwiglu) {
+            float u[8];
+            load(row + k + col, u, valid);
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
-    // amax < 2^E; the digits of v / 2^E in base 128: the first two truncate toward zero (every remainder keeps the sign and is exact in
-    // FP32), the last one rounds to nearest: the rewritten value is within 2^(E-22) of v, without a bias toward zero
-    int exponent = 0;
-    if (amax > 0.f) frexpf(amax, &exponent);
-    exponent = max(exponent, -110);  // 2^(7 - E) and 2^(E - 7) stay finite, normal numbers; runs of denormal-sized values become zeros
-    const float down = ldexpf(1.f, 7 - exponent);
-    uint32_t packed[3] = {0u, 0u, 0u};
+            for (int j = 0; j < 8; ++j) v[j] = silu_times(v[j], u[j]);
+        }
+        if constexpr (ACT == kActGelu) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        float f = v[j] * down;  // |f| < 128
+            for (int j = 0; j < 8; ++j) v[j] = gelu_tanh(v[j]);
+        }
+        if constexpr (ACT == kActRms) {
+            float w[8];
+            if (act_weight) load(act_weight + col, w, valid);
 #pragma unroll
-        for (int p = 0; p < 3; ++p) {
-            const float digit = p < 2 ? truncf(f) : fminf(fmaxf(rintf(f), -127.f), 127.f);
-            packed[p] |= (uint32_t(int(digit)) & 0xffu) << (8 * j);
-            f = (f - digit) * 128.f;
+            for (int j = 0; j < 8; ++j) v[j] = v[j] * inv_rms * (act_weight ? w[j] : 1.f);
+        }
+        float amax = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if constexpr (ACT != kActNone) v[j] = as_float(round_one<T>(v[j]));
+            amax = fmaxf(amax, fabsf(v[j]));
+        }
+#pragma unroll
+        for (int d = 8; d > 0; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));  // of the run: half a warp
+        // amax < 2^E; v / 2^(E-21) rounded to nearest is an integer of 22 bits, its upper 8 the first digit, the two groups of 7 below it the others:
+        // the rewritten value is within 2^(E-22) of v, without a bias.  (E from -110: 2^(7 - E) and 2^(E - 7) stay finite, normal numbers; runs of
+        // denormal-sized values become zeros.)
+        const int exponent = max(int(__float_as_uint(amax) >> 23) - 126, -110);
+        const float down = __uint_as_float(uint32_t(134 - exponent) << 23);
+        uint32_t whole[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) whole[j] = uint32_t(__float2int_rn(v[j] * down * 16384.f));
+        if (col < k) {
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+                const int shift = 14 - 7 * p;
+                const uint32_t mask = p == 0 ? 0xffffffffu : 0x7f7f7f7fu;
+                *reinterpret_cast<uint2*>(digits + int64_t(p * TB + token) * k + col) =
+                    make_uint2(low_bytes(whole[0] >> shift, whole[1] >> shift, whole[2] >> shift, whole[3] >> shift) & mask,
+                               low_bytes(whole[4] >> shift, whole[5] >> shift, whole[6] >> shift, whole[7] >> shift) & mask);
+            }
+            // padding rows of the 8-token layout (24 .. 31): zeros
+            if constexpr (TcShape<TB>::kDigitRows > 3 * TB) *reinterpret_cast<uint2*>(digits + int64_t(3 * TB + token) * k + col) = make_uint2(0u, 0u);
+            if ((lane & 15) == 0) scales[col / kTcRun * TB + token] = amax > 0.f ? __uint_as_float(uint32_t(exponent + 120) << 23) : 0.f;
         }
     }
-#pragma unroll
-    for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(digits + int64_t(p * TB + token) * k + run * kTcRun + 4 * lane) = packed[p];
-    if (lane == 0) scales[run * TB + token] = amax > 0.f ? ldexpf(1.f, exponent - 7) : 0.f;
 }
 
 struct TcParams {
@@ -400,8 +439,9 @@ static TcPlan plan_tc(int m, int n, int k, int sms) {
 }
 
 template <class T, int TB>
-static int launch_tc_shape(const T* x, int64_t ldx, const int8_t* w, const float* sw, const T* bias, const T* residual, const T* rscale, T* y, int m, int n,
-                           int k, const TcPlan& plan, int8_t* digits, float* scales, float* slots, int* counters, cudaStream_t stream) {
+static int launch_tc_shape(const T* x, int64_t ldx, int act, const T* act_weight, float eps, const int8_t* w, const float* sw, const T* bias, const T* residual,
+                           const T* rscale, T* y, int m, int n, int k, const TcPlan& plan, int8_t* digits, float* scales, float* slots, int* counters,
+                           cudaStream_t stream) {
     using S = TcShape<TB>;
     auto kernel = stream_tc<T, TB>;
     static bool configured[64] = {};
@@ -415,8 +455,15 @@ static int launch_tc_shape(const T* x, int64_t ldx, const int8_t* w, const float
     CUtensorMap map_w, map_d;
     if (!make_swizzled_byte_map(&map_w, w, n, k, kTcChannels) || !make_swizzled_byte_map(&map_d, digits, S::kDigitRows, k, S::kDigitRows))
         return int(cudaErrorNotSupported);
-    const int runs = k / kTcRun, units = runs * (TB == 8 ? 16 : TB);
-    const cudaError_t split = launch_after_previous(split_digits<T, TB>, dim3((units + 7) / 8), dim3(256), size_t(0), stream, x, ldx, digits, scales, m, k);
+    const int runs = k / kTcRun, chunk_groups = (k + 8 * kChunk - 1) / (8 * kChunk);
+    const dim3 grid(TB, act == kActRms ? 1 : chunk_groups);
+    static_assert(TcShape<TB>::kDigitRows == 3 * TB || TcShape<TB>::kDigitRows == 4 * TB, "one padding row a token slot, or none");
+    auto splitter = split_digits<T, TB, kActNone>;
+    if (act == kActRms) splitter = split_digits<T, TB, kActRms>;
+    if (act == kActSwiglu) splitter = split_digits<T, TB, kActSwiglu>;
+    if (act == kActGelu) splitter = split_digits<T, TB, kActGelu>;
+    const cudaError_t split =
+        launch_after_previous(splitter, grid, dim3(kRowThreads), size_t(0), stream, x, ldx, act_weight, eps, digits, scales, m, k);
     if (split != cudaSuccess) return int(split);
     TcParams p{scales, sw, bias, residual, rscale, y, slots, counters, m, n, k, (n + kTcChannels - 1) / kTcChannels, runs};
     // behind the split: the stream kernel's set-up and first weight loads run under the split's tail
@@ -424,20 +471,20 @@ static int launch_tc_shape(const T* x, int64_t ldx, const int8_t* w, const float
     return int(launched != cudaSuccess ? launched : cudaGetLastError());
 }
 
-// x (m, K) in T, already transformed; workspace: digits, then scales, then slots (plan sizes, each rounded up to 256 bytes); counters zeroed.
+// x (m, K) in T (SwiGLU: (m, 2 K)); workspace: digits, then scales, then slots (plan sizes, each rounded up to 256 bytes); counters zeroed.
 template <class T>
-static int launch_tc(const void* x, int64_t ldx, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale, void* y, int m,
+static int launch_tc(const void* x, int64_t ldx, int act, const void* act_weight, float eps, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale, void* y, int m,
                      int n, int k, const TcPlan& plan, void* workspace, int* counters, cudaStream_t stream) {
     auto round_up = [](int64_t v) { return (v + 255) / 256 * 256; };
     int8_t* digits = static_cast<int8_t*>(workspace);
     float* scales = reinterpret_cast<float*>(digits + round_up(plan.digit_bytes));
     float* slots = reinterpret_cast<float*>(reinterpret_cast<int8_t*>(scales) + round_up(plan.scale_bytes));
-    auto xs = static_cast<const T*>(x);
+    auto xs = static_cast<const T*>(x), aw = static_cast<const T*>(act_weight);
     auto b = static_cast<const T*>(bias), r = static_cast<const T*>(residual), rs = static_cast<const T*>(rscale);
     auto out = static_cast<T*>(y);
-    if (plan.token_slots == 8) return launch_tc_shape<T, 8>(xs, ldx, w, sw, b, r, rs, out, m, n, k, plan, digits, scales, slots, counters, stream);
-    if (plan.token_slots == 16) return launch_tc_shape<T, 16>(xs, ldx, w, sw, b, r, rs, out, m, n, k, plan, digits, scales, slots, counters, stream);
-    return launch_tc_shape<T, 32>(xs, ldx, w, sw, b, r, rs, out, m, n, k, plan, digits, scales, slots, counters, stream);
+    if (plan.token_slots == 8) return launch_tc_shape<T, 8>(xs, ldx, act, aw, eps, w, sw, b, r, rs, out, m, n, k, plan, digits, scales, slots, counters, stream);
+    if (plan.token_slots == 16) return launch_tc_shape<T, 16>(xs, ldx, act, aw, eps, w, sw, b, r, rs, out, m, n, k, plan, digits, scales, slots, counters, stream);
+    return launch_tc_shape<T, 32>(xs, ldx, act, aw, eps, w, sw, b, r, rs, out, m, n, k, plan, digits, scales, slots, counters, stream);
 }
 
 // What the entry points of stream.cu use.
@@ -449,12 +496,12 @@ int64_t stream_tc_workspace(int m, int n, int k, int sms, int64_t* counter_bytes
     return round_up(plan.digit_bytes) + round_up(plan.scale_bytes) + round_up(plan.slot_bytes);
 }
 
-int stream_tc_launch(const void* x, int64_t ldx, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale, void* y, int m,
+int stream_tc_launch(const void* x, int64_t ldx, int act, const void* act_weight, float eps, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale, void* y, int m,
                      int n, int k, int dtype, int sms, void* workspace, int* counters, cudaStream_t stream) {
     const TcPlan plan = plan_tc(m, n, k, sms);
     if (!plan.token_slots || !workspace || !counters) return -2;
-    if (dtype == 0) return launch_tc<__half>(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, plan, workspace, counters, stream);
-    if (dtype == 1) return launch_tc<bf16>(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, plan, workspace, counters, stream);
+    if (dtype == 0) return launch_tc<__half>(x, ldx, act, act_weight, eps, w, sw, bias, residual, rscale, y, m, n, k, plan, workspace, counters, stream);
+    if (dtype == 1) return launch_tc<bf16>(x, ldx, act, act_weight, eps, w, sw, bias, residual, rscale, y, m, n, k, plan, workspace, counters, stream);
     return -1;
 }
 
