@@ -162,14 +162,15 @@ WQ_DEVICE float magnitude_or_nan(float a, float b) {
     return r;
 }
 template <class T>
-__global__ void __launch_bounds__(256, 5) quantize_blocks_gelu(const T* __restrict__ x, int8_t* __restrict__ q, float* __restrict__ scale, int64_t row0, int k,
-                                                            int64_t ldx, RowShift shift) {
+__global__ void __launch_bounds__(256, 5) quantize_blocks_gelu(const T* __restrict__ x, int8_t* __restrict__ q, float* __restrict__ scale, int64_t row0, uint32_t items,
+                                                               int k, int64_t ldx, RowShift shift) {
     dependents_may_start();
     const int lane = threadIdx.x & 31;
-    const int first = (blockIdx.x * 8 + (threadIdx.x >> 5)) * (kGeluChunks * kChunk);
-    if (first >= k) return;
+    const uint32_t item = blockIdx.x * 8 + (threadIdx.x >> 5), groups = uint32_t(k + kGeluChunks * kChunk - 1) / (kGeluChunks * kChunk);
+    if (item >= items) return;
+    const int first = int(item % groups) * (kGeluChunks * kChunk);
     const int kblocks = (k + kBlockK - 1) / kBlockK;
-    const int64_t row = row0 + blockIdx.y;
+    const int64_t row = row0 + item / groups;
     const T* src = first_row(x, ldx, shift) + row * ldx + first + lane * 8;
     uint4 raw[kGeluChunks];
 #pragma unroll
@@ -640,12 +641,23 @@ static int launch_blocks(const void* x, int8_t* q, float* scale, int m, int k, i
         else if (k <= 16384) quantize_blocks_rms<T, GROUP, 8><<<m, kRowThreads, 0, stream>>>(src, q, scale, m, k, ldx, aw, eps, shift);
         else quantize_blocks_rms<T, GROUP, 0><<<m, kRowThreads, 0, stream>>>(src, q, scale, m, k, ldx, aw, eps, shift);
     } else {
-        constexpr bool kGelu = ACT == kActGelu && GROUP == 0;  // (a rotation needs every accurate value)
-        const int chunks = (k + kChunk - 1) / kChunk, per_cta = 8 * (kGelu ? kGeluChunks : 1);
+        const int chunks = (k + kChunk - 1) / kChunk;
+        if constexpr (ACT == kActGelu && GROUP == 0) {  // (a rotation needs every accurate value)
+            // Four chunks a warp want enough warps: 20 an SM (BF16, 5888 values a row, one chunk a warp with tanhf and this, us: 256 rows 4.0
+            // and 4.5, 512 5.9 and 5.7, 1560 14.0 and 10.9).
+            const int64_t groups = (chunks + kGeluChunks - 1) / kGeluChunks;
+            if (m * groups >= 3000) {
+                const int64_t most = (int64_t(1) << 30) / groups;
+                for (int64_t row0 = 0; row0 < m; row0 += most) {
+                    const uint32_t items = uint32_t((m - row0 < most ? m - row0 : most) * groups);
+                    quantize_blocks_gelu<T><<<(items + 7) / 8, 256, 0, stream>>>(src, q, scale, row0, items, k, ldx, shift);
+                }
+                return int(cudaGetLastError());
+            }
+        }
         for (int64_t row0 = 0; row0 < m; row0 += 65535) {
-            const dim3 grid((chunks + per_cta - 1) / per_cta, unsigned(m - row0 < 65535 ? m - row0 : 65535));
+            const dim3 grid((chunks + 7) / 8, unsigned(m - row0 < 65535 ? m - row0 : 65535));
             if constexpr (GROUP > 0 && ACT == kActNone) quantize_blocks_rotated<T, GROUP><<<dim3((chunks + 15) / 16, grid.y), 256, 0, stream>>>(src, q, scale, row0, k, ldx, shift);
-            else if constexpr (kGelu) quantize_blocks_gelu<T><<<grid, 256, 0, stream>>>(src, q, scale, row0, k, ldx, shift);
             else quantize_blocks_items<T, GROUP, ACT><<<grid, 256, 0, stream>>>(src, q, scale, row0, k, ldx, shift);
         }
     }
@@ -682,8 +694,8 @@ static int launch_rows(const void* x, int8_t* hi, int8_t* lo, float* scale, int 
     auto src = static_cast<const T*>(x);
     auto aw = static_cast<const T*>(act_weight);
     // (rms_norm: the order of the row's sum is that of eight values a lane; gelu and swiglu: how their last product and the rotation's first sum
-    // are fused is that kernel's)
-    if constexpr (GROUP > 0 && ACT == kActNone) {
+    // are fused is that kernel's; groups of 16 with a low part: two more digits' worth of registers for twelve shuffles, 1560 x 13824 19.9 -> 25.0 us)
+    if constexpr (GROUP > 0 && ACT == kActNone && !(GROUP == 16 && HILO)) {
         if (k <= 16384) {
             const int chunks = (k + kChunk - 1) / kChunk, per_half = k <= 4096 ? 1 : k <= 8192 ? 2 : 4;
             const int threads = 32 * ((chunks + 2 * per_half - 1) / (2 * per_half));
