@@ -447,3 +447,22 @@ def test_k_split_is_refused_where_it_does_not_fit(wq):
     for rows, channels, k in ((129, 256, 512), (64, 20000, 512), (64, 256, 128)):  # rows, channels for the GPU's clusters, blocks of K
         with pytest.raises(RuntimeError, match="-2"):
             wq.gemm(a[:rows, :k].contiguous(), None, sa[:rows], b[:channels, :k].contiguous(), sb[:channels], None, torch.bfloat16, 0, 40)
+
+
+@pytest.mark.parametrize("mode,variants", [("exact+g", (24, 19)), ("block+g", (13, 18))])
+@pytest.mark.parametrize("shape", [(1, 8, 128), (100, 264, 1040), (333, 1023, 640 + 16), (1024, 1536, 1152)], ids=str)
+def test_group_scales_gathered_or_regrouped(wq, shape, mode, variants):
+    """Tiles of up to 128 columns take the group scales of few rows as the caller holds them; the same rows as part of a longer input have them
+    regrouped first.  The same bits, and the oracle's values."""
+    m, n, k = shape
+    dtype = torch.float16
+    base, a, a_lo, sa, b, sb, bias, res, rs = operands(mode, m, n, k, dtype, 36, True)
+    dev = lambda t: None if t is None else t.cuda()
+    longer = lambda t: None if t is None else torch.cat([t, torch.zeros(1100, *t.shape[1:], dtype=t.dtype)]).cuda()
+    expected = oracle.gemm(base, a.numpy(), None if a_lo is None else a_lo.numpy(), sa.numpy(), b.numpy(), sb.numpy(), bias, res, rs, dtype)
+    for variant in variants:
+        y = wq.gemm(dev(a), dev(a_lo), dev(sa), dev(b), dev(sb), dev(bias), dtype, 0, variant, residual=dev(res), residual_scale=dev(rs))
+        assert rel(y, expected) < 1e-3
+        whole = wq.gemm(longer(a), longer(a_lo), longer(sa), dev(b), dev(sb), dev(bias), dtype, 0, variant, residual=longer(res), residual_scale=dev(rs))
+        assert torch.equal(whole[:m], y)
+    assert wq.debug_status() == 0

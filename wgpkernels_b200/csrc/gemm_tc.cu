@@ -73,6 +73,7 @@ template <int MODE, int BN, bool WIDE, int PARTS, bool PAIR> struct Shape {
     static constexpr int kChunk = PARTS == 2 ? 32 : kWGroup && BN == 256 ? 8 : 16;
     static_assert(!(kWGroup && PARTS == 2 && BN == 256), "block+g on 256 columns needs sixteen drain warps");
     static constexpr int kRingBytes = kWGroup ? kScaleRing * BN * 4 : 0;
+    static constexpr bool kGatherScales = kWGroup && BN <= 128;  // may take the group scales as the caller holds them (256 columns: too few registers)
     // Output staging: every drain warp owns one buffer of 32 rows x 32 columns of 16-bit outputs (2 KiB, 64-byte swizzle) from which the
     // TMA unit writes whole 64-byte row segments.  kWide (several destinations): 32 rows x 64 columns (4 KiB, 128-byte swizzle), so that
     // rows of 128 bytes cross NVLink; one operand stage less fits then.
@@ -456,13 +457,27 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                     const int params_after = (kblocks < 2 ? kblocks : 2) - 1;
                     for (int kb = 0; kb < kblocks && ok; ++kb) {
                         if (!(ok = whole_warp(wait_on(bar_ring_empty + 8 * slot, phase ^ 1u, abort_flag, kTimeoutScales)))) break;
-                        // the tile's BN scales of this block are contiguous in sb_blocks: one bulk copy, up to kScaleRing of them in flight
-                        if (lane == 0) {
-                            mbar_expect_tx(bar_ring_full + 8 * slot, BN * 4);
-                            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                                             smem_u32(scale_ring + slot * BN)),
-                                         "l"(p.sb_blocks + int64_t(kb) * p.n_pad + c.n0), "r"(BN * 4), "r"(bar_ring_full + 8 * slot)
-                                         : "memory");
+                        if (!S::kGatherScales || p.sb_blocks) {
+                            // the tile's BN scales of this block are contiguous in sb_blocks: one bulk copy, up to kScaleRing of them in flight
+                            if (lane == 0) {
+                                mbar_expect_tx(bar_ring_full + 8 * slot, BN * 4);
+                                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                                 smem_u32(scale_ring + slot * BN)),
+                                             "l"(p.sb_blocks + int64_t(kb) * p.n_pad + c.n0), "r"(BN * 4), "r"(bar_ring_full + 8 * slot)
+                                             : "memory");
+                            }
+                        } else {
+                            // a column a lane, from where the caller holds them: kblocks scales a column, so eight blocks come with one sector
+                            float gathered[BN / 32];
+#pragma unroll
+                            for (int i = 0; i < BN / 32; ++i) {
+                                const int col = c.n0 + lane + 32 * i;
+                                gathered[i] = col < p.n ? p.sb[0][int64_t(col) * kblocks + kb] : 0.f;
+                            }
+#pragma unroll
+                            for (int i = 0; i < BN / 32; ++i) scale_ring[slot * BN + lane + 32 * i] = gathered[i];
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(bar_ring_full + 8 * slot);
                         }
                         if (++slot == kScaleRing) { slot = 0; phase ^= 1u; }
                         if (kb == params_after) ok = stage_params(c);
@@ -1022,6 +1037,12 @@ struct GemmArgs {
 // Rows a tensor map of a row window may address: the window's position is only known on the GPU.
 constexpr int64_t kUnboundedRows = int64_t(1) << 30;
 
+// Group scales of tiles of up to 128 columns: few rows (a few tiles a CTA) have them gathered by the kernel, a column a lane, instead of regrouped by
+// a launch of their own.  Measured (regrouping and GEMM, L2 cold, regrouped -> gathered, us): exact+g 333 x 12280 x 3008 36.9 -> 35.1, 100 x 4096 x
+// 4096 20.1 -> 17.9, 1024 x 4096 x 4096 44.7 -> 44.5, 2048 x 8192 x 4096 139.4 -> 141.0; block+g 100 x 4096 x 4096 17.7 -> 17.1, 48 x 2048 x 14336
+// 45.5 -> 46.4 (its drain is done with a block sooner than a gather of all columns comes back).
+static bool gathers_scales(const GemmArgs& g, bool hilo) { return g.m <= 1024 && (hilo || g.k <= 8192); }
+
 template <class T, int MODE, int BN, bool WIDE, bool DUMP, int PARTS, bool PAIR = false>
 static int launch(const GemmArgs& g, cudaStream_t stream) {
     using S = Shape<MODE, BN, WIDE, PARTS, PAIR>;
@@ -1074,8 +1095,8 @@ static int launch(const GemmArgs& g, cudaStream_t stream) {
     p.seg_tiles = (g.n + BN - 1) / BN;
     p.tiles_n = p.seg_tiles * g.segments;
     p.window = g.window;
-    if (S::kWGroup) {
-        if (!g.scale_scratch || (reinterpret_cast<uintptr_t>(g.scale_scratch) & 15)) return -2;
+    if (S::kWGroup && (!g.scale_scratch || (reinterpret_cast<uintptr_t>(g.scale_scratch) & 15))) return -2;
+    if (S::kWGroup && !(S::kGatherScales && gathers_scales(g, S::kHilo))) {
         const int kblocks = (g.k + kStageK - 1) / kStageK;
         p.n_pad = padded_n(g.n);
         p.sb_blocks = g.scale_scratch;
