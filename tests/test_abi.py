@@ -218,7 +218,7 @@ def test_few_token_arguments(lib):
 
     assert call(m=0) == 0
     assert call(dtype=2) == -1
-    assert call(m=33) == call(k=1024) == call(k=4096 + 64) == call(act=1) == call(act=7) == -2
+    assert call(m=33) == call(k=1024) == call(k=4096 + 64) == call(act=1) == call(act=7) == -2  # (1024, rms_norm: with scratch only)
     assert call(x=odd) == call(w=odd) == call(ldx=4098) == -2
     # more than four tokens: scratch of wq8_small, 16-byte aligned rows and norm weights
     assert call(m=16) == call(m=16, slots=one, counters=one) == call(m=16, slots=scratch) == -2

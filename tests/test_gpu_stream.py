@@ -188,16 +188,17 @@ def test_input_operation_and_stream_in_one_launch(wq, m, shape, act, dtype):
 def test_how_the_shapes_run(wq):
     takes = wq._require().wq8_few_takes
     assert [takes(m, 4096, 4096, 0, 148) for m in (1, 2, 3, 4, 5, 32, 33)] == [1, 1, 1, 1, 2, 2, 0]
-    assert [takes(1, 4096, k, 0, 148) for k in (1024, 2048, 2048 + 64, 16384, 16384 + 128)] == [0, 1, 0, 1, 0]
-    assert [takes(1, 4096, 4096, act, 148) for act in (0, 1, 2, 3, 4)] == [1, 0, 1, 1, 0]
+    assert [takes(1, 4096, k, 0, 148) for k in (1024, 2048, 2048 + 64, 16384, 16384 + 128)] == [2, 1, 0, 1, 2]
+    assert [takes(3, 4096, k, 0, 148) for k in (4096, 4096 + 128)] == [1, 2]
+    assert [takes(1, 4096, 4096, act, 148) for act in (0, 1, 2, 3, 4)] == [1, 2, 1, 1, 0]
     assert [takes(9, 4096, k, act, 148) for act in (0, 1, 2, 3) for k in (128, 4096, 4096 + 64)] == [2, 2, 0] * 4
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
 @pytest.mark.parametrize("act", [None, "rms_norm", "swiglu", "gelu"])
-@pytest.mark.parametrize("m,n,k", [(5, 40, 128), (8, 1000, 1152), (9, 264, 4096 + 128), (16, 2048, 14336), (17, 129, 2048), (32, 520, 5120)], ids=str)
-def test_input_operation_in_the_digit_split(wq, m, n, k, act, dtype):
-    """wq8_few above four tokens: the digits of op(x) rounded as transform_rows rounds it, so the bits of wq8_small on those rows."""
+@pytest.mark.parametrize("m,n,k", [(2, 264, 1024), (4, 1000, 6144 + 128), (5, 40, 128), (8, 1000, 1152), (9, 264, 4096 + 128), (16, 2048, 14336), (17, 129, 2048), (32, 520, 5120)], ids=str)
+def test_input_operation_in_the_digit_split(wq, m, n, k, act, dtype, monkeypatch):
+    """wq8_few in two launches: the digits of op(x) rounded as transform_rows rounds it, so the bits of wq8_small on those rows."""
     _, w, sw, bias, res, rs = case(m, n, k, dtype, 151, True)
     x = randn((m, 2 * k if act == "swiglu" else k), dtype, 152)
     x[:, ::131] *= 60
@@ -205,6 +206,7 @@ def test_input_operation_in_the_digit_split(wq, m, n, k, act, dtype):
     norm = (1 + 0.1 * randn((k,), torch.float32, 153)).to(dtype) if act == "rms_norm" else None
     gx, gw, gsw, gbias, gres, grs, gnorm = cuda(x, w, sw, bias, res, rs, norm)
     prepared = wq.transform_rows(gx, 0, act, gnorm, 1e-6) if act else gx
+    monkeypatch.setattr(wq, "_stream_planes", lambda *args: False)  # wq8_small for any number of tokens
     expected = wq.small(prepared, gw, gsw, gbias, gres, grs)
     target = gres.clone()
     y = wq.linear(gx, gw, gsw, gbias, mode="small", act=act, act_weight=gnorm, eps=1e-6, residual=target, residual_scale=grs, out=target)

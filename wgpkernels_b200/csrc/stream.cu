@@ -829,10 +829,10 @@ static int64_t tensor_core_scratch(int m, int n, int k, int sms, int64_t* counte
 }
 
 // The few-token linear with its input operation: up to four tokens in one launch where the digits of all of K fit beside the weight rings
-// (stream_few.cu; not behind rms_norm, whose row sum comes first), more in two, the input operation being part of the digit split.
+// (stream_few.cu; not behind rms_norm, whose row sum comes first), else in two, the input operation being part of the digit split.
 WQ_API int wq8_few_takes(int m, int n, int k, int act, int sms) {
     if (act < kActNone || act > kActGelu) return 0;
-    if (m <= 4) return act != kActRms && wq8_stream_planes_workspace(m, n, k, sms) > 0 && stream_few_takes(m, k);
+    if (m <= 4 && act != kActRms && wq8_stream_planes_workspace(m, n, k, sms) > 0 && stream_few_takes(m, k)) return 1;
     int64_t counter_bytes = 0;
     return tensor_core_scratch(m, n, k, sms, &counter_bytes) ? 2 : 0;
 }
