@@ -466,3 +466,25 @@ def test_group_scales_gathered_or_regrouped(wq, shape, mode, variants):
         whole = wq.gemm(longer(a), longer(a_lo), longer(sa), dev(b), dev(sb), dev(bias), dtype, 0, variant, residual=longer(res), residual_scale=dev(rs))
         assert torch.equal(whole[:m], y)
     assert wq.debug_status() == 0
+
+
+@pytest.mark.parametrize("mode,staged,loaded", [("block", (10, 16), 20), ("block+g", (12,), 18)])
+@pytest.mark.parametrize("shape", [(1, 8, 128), (129, 264, 128), (257, 520, 640 + 16), (300, 2304, 1152), (2431, 5120, 384)], ids=str)
+def test_residual_through_the_staging_tiles(wq, shape, mode, staged, loaded):
+    """The residual that the TMA unit brings in ahead of the write-out and the one that the threads load: the same bits, in place or not, as a column
+    range of a wider matrix; one block of K, partial tiles in both directions, several tiles a CTA."""
+    m, n, k = shape
+    dtype = torch.bfloat16 if m % 2 else torch.float16
+    _, a, _, sa, b, sb, bias, res, rs = operands(mode, m, n, k, dtype, 37, True)
+    a, sa, b, sb, bias, res, rs = (t.cuda() for t in (a, sa, b, sb, bias, res, rs))
+    call = lambda variant, **kw: wq.gemm(a, None, sa, b, sb, bias, dtype, 0, variant, residual_scale=rs, **kw)
+    expected = call(loaded, residual=res)
+    wide = torch.zeros(m, n + 24, dtype=dtype, device="cuda")
+    wide[:, 8:8 + n] = res
+    for variant in staged:
+        assert torch.equal(call(variant, residual=res), expected)
+        target = res.clone()
+        assert torch.equal(call(variant, residual=target, out=target), expected)
+        if n % 8 == 0:
+            assert torch.equal(call(variant, residual=wide[:, 8:8 + n], out=torch.empty_like(res)), expected)
+    assert wq.debug_status() == 0

@@ -3,7 +3,8 @@
 //
 //   warp 0      TMA producer: A (and A_lo) 128 x 128-byte tiles, B BN x 128-byte tiles, 128-byte swizzle, ring of kStages buffers
 //   warps 1-2   MMA issue (the whole warp runs the loop, one elected lane issues): 4 (x2 with a low part) tcgen05.mma of K = 32 per stage; warp 2 owns tensor memory
-//   warp 3      column parameters of the tile being finished (and the per-block weight scales of group-scaled weights) into shared memory
+//   warp 3      column parameters of the tile being finished (and the per-block weight scales of group-scaled weights) into shared memory; block,
+//               block+g: its residual as well, through TMA
 //   warps 4-19  drain: 16 warps, warp w reads tensor-memory lanes 32 (w % 4) .. + 32 and a quarter of the tile's columns: tcgen05.ld of the
 //               INT32 sums, conversion and promotion to FP32 (two-wide FP32 FMAs), bias / residual, one rounding, TMA stores
 //
@@ -79,7 +80,16 @@ template <int MODE, int BN, bool WIDE, int PARTS, bool PAIR> struct Shape {
     // rows of 128 bytes cross NVLink; one operand stage less fits then.
     static constexpr bool kWide = WIDE && kEpiColumns >= 64;
     static constexpr int kStoreTile = kWide ? 32 * 64 * 2 : 32 * 32 * 2;
-    static constexpr int kStoreBytes = kDrainWarps * kStoreTile;
+    // Per-block modes on sixteen drain warps: a staging tile for each chunk of 32 columns, so that a chunk does not wait for the store of the one
+    // before it, and the residual comes through them: warp 3 has the TMA unit bring a tile's residual into the staging tiles, idle while
+    // the blocks are drained, and the outputs are written over it.  (Fetched by the drain threads at the write-out, 64 bytes of 32 rows a
+    // warp, it took 5000 clocks for the first chunk and 3100 for the second; a chunk without a residual takes 1200.)  Measured with a residual, us:
+    // block 32760 x 5120 x 13824 2312 -> 2235, block+g 16384 x 12288 x 3072 1052 -> 964, block on 128 channels 1024 x 5120 x 5120 56.2 ->
+    // 52.3; without one 0 to 0.7 % faster.  Tiles of 128 columns with group scales keep the loads: warp 3 is busy with the scales of short blocks
+    // (block+g 1024 x 4096 x 4096 49.7 -> 58.4, exact+g 4096 x 4096 x 4096 4 % slower).
+    static constexpr bool kTmaResidual = PARTS == 4 && !WIDE && (MODE == kBlock || (MODE == kBlockG && BN == 256));
+    static constexpr int kStoreTiles = kTmaResidual ? kEpiColumns / 32 : 1;  // of a drain warp
+    static constexpr int kStoreBytes = kDrainWarps * kStoreTiles * kStoreTile;
     // Column parameters of the tile being finished (weight scale and bias as FP32, residual scale in the output type), shared by the drain warps.
     static constexpr int kParamBytes = BN * 10;
     static constexpr int kBarrierBytes = 384;
@@ -136,7 +146,7 @@ struct GemmParams {
 // peers (ordinary TMA stores over NVLink; nothing is ever loaded from a peer).  With segments: map s = the output of weight s.
 constexpr int kMaxDestinations = 8;
 struct OutputMaps { CUtensorMap map[kMaxDestinations]; };
-struct InputMaps { CUtensorMap a, a_lo, a_tail, a_lo_tail; };
+struct InputMaps { CUtensorMap a, a_lo, a_tail, a_lo_tail, residual; };  // residual: boxes of 32 rows x 32 columns, as the outputs
 struct WeightMaps { CUtensorMap map[kMaxSegments]; };
 
 struct TileCoord { int m0, n0, segment; };
@@ -185,16 +195,17 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
     float* param_sb = reinterpret_cast<float*>(params);
     float* param_bias = reinterpret_cast<float*>(params + BN * 4);
     T* param_rscale = reinterpret_cast<T*>(params + BN * 8);
+    const auto staged_residual = [&]() { return S::kTmaResidual && p.residual && p.tma_y; };  // (asked for where it counts, not kept in a register)
     uint64_t* bars = reinterpret_cast<uint64_t*>(params + S::kParamBytes);
     // barrier layout: full[6], empty[6], acc_full[4], acc_empty[4], ring_full[kScaleRing], ring_empty[kScaleRing], params_written,
-    // params_consumed; then the TMEM slot and the abort flag
+    // params_consumed, staging_free, residual; then the TMEM slot and the abort flag
     constexpr int kMaxStages = 6, kMaxAcc = 4;
     static_assert(kAccBuffers <= kMaxAcc && kStages <= kMaxStages, "barrier table");
     const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * kMaxStages, bar_acc_full = bar_empty + 8 * kMaxStages,
                    bar_acc_empty = bar_acc_full + 8 * kMaxAcc, bar_ring_full = bar_acc_empty + 8 * kMaxAcc,
                    bar_ring_empty = bar_ring_full + 8 * kScaleRing, bar_params_written = bar_ring_empty + 8 * kScaleRing,
-                   bar_params_consumed = bar_params_written + 8;
-    static_assert(8 * (2 * kMaxStages + 2 * kMaxAcc + 2 * kScaleRing + 2) <= S::kBarrierBytes - 32, "barriers overlap the TMEM slot");
+                   bar_params_consumed = bar_params_written + 8, bar_staging_free = bar_params_consumed + 8, bar_residual = bar_staging_free + 8;
+    static_assert(8 * (2 * kMaxStages + 2 * kMaxAcc + 2 * kScaleRing + 4) <= S::kBarrierBytes - 32, "barriers overlap the TMEM slot");
     uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(bars) + S::kBarrierBytes - 32);
     int& abort_word = *reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(bars) + S::kBarrierBytes - 28);
     volatile int* abort_flag = &abort_word;
@@ -222,6 +233,8 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
         }
         mbar_init(bar_params_written, 32);
         mbar_init(bar_params_consumed, kDrainWarps);
+        mbar_init(bar_staging_free, kDrainWarps);
+        mbar_init(bar_residual, 1);
         for (int s = 0; s < kScaleRing; ++s) {
             mbar_init(bar_ring_full + 8 * s, 1);
             mbar_init(bar_ring_empty + 8 * s, kDrainWarps);
@@ -433,6 +446,21 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
             int slot = 0, tile_count = 0;
             uint32_t phase = 0;
             bool ok = true;
+            // The residual of the tile in hand, once every drain warp's stores of the tile before it have left the staging tiles: a box a lane.
+            [[maybe_unused]] int residual_tiles = 0;
+            [[maybe_unused]] auto stage_residual = [&](const TileCoord& c) -> bool {
+                if (!staged_residual()) return true;
+                if (!whole_warp(wait_on(bar_staging_free, uint32_t(residual_tiles) & 1u, abort_flag, kTimeoutParams))) return false;
+                ++residual_tiles;
+                if (lane == 0) mbar_expect_tx(bar_residual, S::kStoreBytes);
+                __syncwarp();
+                if (lane < kDrainWarps * S::kStoreTiles) {
+                    const int drain_warp = lane / S::kStoreTiles, chunk = lane % S::kStoreTiles;
+                    tma_load_2d(store_stage + lane * S::kStoreTile, &in_maps.residual, bar_residual, c.n0 + (drain_warp >> 2) * kEpi + chunk * 32,
+                                c.m0 + (drain_warp & 3) * 32);
+                }
+                return true;
+            };
             auto stage_params = [&](const TileCoord& c) -> bool {
                 if (!p.vector_io) return true;
                 // every drain warp is done with the previous tile's parameters
@@ -455,6 +483,8 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                 if constexpr (S::kWGroup) {
                     // the first two blocks' scales go first: the drain warps start on them right after the previous tile's write-out
                     const int params_after = (kblocks < 2 ? kblocks : 2) - 1;
+                    // (the drain warps report their staging tiles free after two blocks: by then they need the scales of no block past the ring)
+                    [[maybe_unused]] const int residual_after = (kblocks < kScaleRing ? kblocks : kScaleRing) - 1;
                     for (int kb = 0; kb < kblocks && ok; ++kb) {
                         if (!(ok = whole_warp(wait_on(bar_ring_empty + 8 * slot, phase ^ 1u, abort_flag, kTimeoutScales)))) break;
                         if (!S::kGatherScales || p.sb_blocks) {
@@ -481,11 +511,18 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                         }
                         if (++slot == kScaleRing) { slot = 0; phase ^= 1u; }
                         if (kb == params_after) ok = stage_params(c);
+                        if constexpr (S::kTmaResidual) {
+                            if (ok && kb == residual_after) ok = stage_residual(c);
+                        }
                     }
                 } else {
                     ok = stage_params(c);
+                    if constexpr (S::kTmaResidual) {
+                        if (ok) ok = stage_residual(c);
+                    }
                 }
             }
+            if (S::kTmaResidual && !ok) await_issued_fills(bar_residual, 1, uint32_t(residual_tiles) & 1u);
         }
     }
     } else {
@@ -501,7 +538,7 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
         uint32_t buffer_phases = 0;         // per-block modes: bit b = phase of buffer b's next use
         bool ok = true;
         const int drain_warp = warp - kControlWarps;
-        const uint32_t my_stage = store_stage + drain_warp * S::kStoreTile;
+        const uint32_t my_stage = store_stage + drain_warp * S::kStoreTiles * S::kStoreTile;
         int tile_count = 0;  // tiles this CTA has finished: the phase of the parameter hand-over barriers
         float sa_ahead[2] = {0.f, 0.f};
         bool sa_ahead_valid = false;
@@ -611,7 +648,7 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                 const T* bias = static_cast<const T*>(p.bias[c.segment]);
 #pragma unroll
                 for (int part16 = 0; part16 < 32; part16 += 16) {
-                    float* mine = store_stage_generic + (drain_warp * S::kStoreTile + lane * 64) / 4;
+                    float* mine = store_stage_generic + (drain_warp * S::kStoreTiles * S::kStoreTile + lane * 64) / 4;
 #pragma unroll
                     for (int j = 0; j < 16; ++j) mine[j] = v[part16 + j];
 #pragma unroll 1
@@ -638,18 +675,31 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
             // for the TMA unit to be done reading the staging tile of the previous chunk, so that wait hides behind the arithmetic.
             // Same operations per output, in the same order, as `emit`: the bits do not depend on which of the two writes a tile.
             const bool fast_tile = !S::kWide && p.vector_io && p.tma_y && p.destinations == 1 && c.n0 + BN <= p.n && !(rscale && p.window.span);
-            // 16-byte piece g of the 32 residual values that belong to chunk `chunk` of this thread's row (plain loads: y may be the residual).  For
-            // block+g on 256 channels a piece is fetched where it is added: four at once spill.
-            const T* res_row = residual && row_ok ? residual + (out_shift + row) * p.ld_residual + col0 : nullptr;
-            constexpr bool kResidualByPiece = MODE == kBlockG && BN == 256;
-            auto fetch_residual_piece = [&](int chunk, int g) { return *reinterpret_cast<const uint4*>(res_row + chunk * 32 + 8 * g); };
+            // The residual: 16-byte pieces of this thread's row with plain loads (y may be the residual), or from the staging tile that the chunk's outputs
+            // will be written to (row `lane`, piece g at its place in the 64-byte swizzle).
+            const T* res_row = !S::kTmaResidual && residual && row_ok ? residual + (out_shift + row) * p.ld_residual + col0 : nullptr;
             auto fetch_residual = [&](int chunk, uint4* res) {
 #pragma unroll
-                for (int g = 0; g < 4; ++g) res[g] = fetch_residual_piece(chunk, g);
+                for (int g = 0; g < 4; ++g) res[g] = *reinterpret_cast<const uint4*>(res_row + chunk * 32 + 8 * g);
+            };
+            auto staged_piece = [&](int chunk, int g) {
+                return my_stage + (S::kStoreTiles > 1 ? chunk * S::kStoreTile : 0) + lane * 64 + (uint32_t(g) ^ ((uint32_t(lane) >> 1) & 3u)) * 16;
             };
             auto emit_fast = [&](const float2* a, int chunk, const uint4* res, bool has_res) {
                 const int ct = part * kEpi + chunk * 32;  // first column of the chunk within the tile
-                uint32_t packed[16];
+                // The TMA store that last read the staging tile must be done with it.  Of two tiles that is the store before last: over, so the outputs go
+                // there as they come (fewer registers); of one, it is awaited behind the arithmetic.
+                auto staging_free = [&]() {
+                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(S::kStoreTiles - 1) : "memory");
+                    __syncwarp();
+                };
+                constexpr bool kAtOnce = S::kStoreTiles > 1;
+                auto stage_piece = [&](int g, const uint32_t* pairs) {
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(staged_piece(chunk, g)), "r"(pairs[0]), "r"(pairs[1]), "r"(pairs[2]), "r"(pairs[3])
+                                 : "memory");
+                };
+                if constexpr (kAtOnce) staging_free();
+                uint32_t packed[kAtOnce ? 4 : 16];
 #pragma unroll
                 for (int g = 0; g < 4; ++g) {  // eight columns
                     float2 o[4];
@@ -671,7 +721,10 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                         }
                     }
                     if (has_res) {
-                        const uint4 res_g = kResidualByPiece ? fetch_residual_piece(chunk, g) : res[g];
+                        uint4 res_g;
+                        if constexpr (S::kTmaResidual)
+                            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(res_g.x), "=r"(res_g.y), "=r"(res_g.z), "=r"(res_g.w) : "r"(staged_piece(chunk, g)) : "memory");
+                        else res_g = res[g];
                         const uint4 rs = *reinterpret_cast<const uint4*>(param_rscale + ct + 8 * g);
                         const uint32_t rs_raw[4] = {rs.x, rs.y, rs.z, rs.w}, res_raw[4] = {res_g.x, res_g.y, res_g.z, res_g.w};
 #pragma unroll
@@ -683,24 +736,20 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                         }
                     }
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) packed[4 * g + e] = pack_pair<T>(o[e].x, o[e].y);
+                    for (int e = 0; e < 4; ++e) packed[(kAtOnce ? 0 : 4 * g) + e] = pack_pair<T>(o[e].x, o[e].y);
+                    if constexpr (kAtOnce) stage_piece(g, packed);
                 }
-                // the TMA store that last read this warp's staging tile must be done with it
-                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                __syncwarp();
+                if constexpr (!kAtOnce) {
+                    staging_free();
 #pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    // row `lane` of the staging tile, 16-byte piece g at its place in the 64-byte swizzle
-                    const uint32_t piece = uint32_t(g) ^ ((uint32_t(lane) >> 1) & 3u);
-                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(my_stage + lane * 64 + piece * 16), "r"(packed[4 * g]),
-                                 "r"(packed[4 * g + 1]), "r"(packed[4 * g + 2]), "r"(packed[4 * g + 3])
-                                 : "memory");
+                    for (int g = 0; g < 4; ++g) stage_piece(g, packed + 4 * g);
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) {
                     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(&out_maps.map[c.segment]),
-                                 "r"(c.n0 + ct), "r"(c.m0 + quarter * 32), "r"(my_stage)
+                                 "r"(c.n0 + ct), "r"(c.m0 + quarter * 32),
+                                 "r"(my_stage + (S::kStoreTiles > 1 ? chunk * S::kStoreTile : 0))
                                  : "memory");
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 }
@@ -839,6 +888,12 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                     if constexpr (kAccBuffers > 1) if (ok && kb + 1 < kblocks) ok = drain_block(std::integral_constant<int, 1>(), kb + 1);
                     if constexpr (kAccBuffers > 2) if (ok && kb + 2 < kblocks) ok = drain_block(std::integral_constant<int, 2>(), kb + 2);
                     if constexpr (kAccBuffers > 3) if (ok && kb + 3 < kblocks) ok = drain_block(std::integral_constant<int, 3>(), kb + 3);
+                    if constexpr (S::kTmaResidual && !DUMP) {
+                        if (kb == 0 && lane == 0 && staged_residual()) {  // the stores of the tile before have been read by now: no wait
+                            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                            mbar_arrive(bar_staging_free);
+                        }
+                    }
                 }
                 if (PARTS == 4) ok = whole_warp(*abort_flag == 0);
                 if (!ok) break;
@@ -856,6 +911,7 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                 }
                 if constexpr (!DUMP) {
                     if (!(ok = await_params())) break;
+                    if (staged_residual() && !(ok = whole_warp(wait_on(bar_residual, uint32_t(tile_count) & 1u, abort_flag, kTimeoutParams)))) break;
                     if (fast_tile) {
                         // the residual of a chunk is requested while the chunk before it is written out, where the registers allow it
                         constexpr bool kResidualAhead = PARTS == 2 && !S::kWGroup;
@@ -867,8 +923,8 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
                                 if (res_row && chunk + 1 < kEpi / 32) fetch_residual(chunk + 1, res[(chunk + 1) & 1]);
                                 emit_fast(&accf[chunk * 16], chunk, res[chunk & 1], res_row != nullptr);
                             } else {
-                                if (!kResidualByPiece && res_row) fetch_residual(chunk, res[0]);
-                                emit_fast(&accf[chunk * 16], chunk, res[0], res_row != nullptr);
+                                if (!S::kTmaResidual && res_row) fetch_residual(chunk, res[0]);
+                                emit_fast(&accf[chunk * 16], chunk, res[0], S::kTmaResidual ? staged_residual() : res_row != nullptr);
                             }
                         }
                     } else
@@ -1064,7 +1120,7 @@ static int launch(const GemmArgs& g, cudaStream_t stream) {
     const int64_t a_rows = windowed ? kUnboundedRows : g.m;
     p.tail_rows = windowed ? g.m % kBM : 0;
     if (!make_map(&in_maps.a, g.a, a_rows, g.k, kBM)) return int(cudaErrorNotSupported);
-    in_maps.a_lo = in_maps.a_tail = in_maps.a_lo_tail = in_maps.a;
+    in_maps.a_lo = in_maps.a_tail = in_maps.a_lo_tail = in_maps.residual = in_maps.a;
     if (S::kHilo && !make_map(&in_maps.a_lo, g.a_lo, a_rows, g.k, kBM)) return int(cudaErrorNotSupported);
     if (p.tail_rows) {
         if (!make_map(&in_maps.a_tail, g.a, a_rows, g.k, p.tail_rows)) return int(cudaErrorNotSupported);
@@ -1120,6 +1176,8 @@ static int launch(const GemmArgs& g, cudaStream_t stream) {
             out_maps.map[d] = in_maps.a;
     }
     if (p.destinations > 1 && !p.tma_y) return -2;  // several destinations are only written by the TMA stores
+    if (S::kTmaResidual && p.tma_y && g.residual && !make_output_map(&in_maps.residual, g.residual, g.m, g.n, p.ld_residual, std::is_same<T, bf16>::value, false))
+        return int(cudaErrorNotSupported);
     const int64_t tiles = int64_t(p.tiles_m) * p.tiles_n;
     const int sms = g.sms > 0 ? g.sms : 148;
     if (PAIR && windowed) return -2;  // a row window's last tile is fetched through a narrower map: single CTAs only
