@@ -1,0 +1,71 @@
+"""The native host side of the two whole-linear library calls: which calls it takes, and that the others go the general way with the same bits."""
+import pytest
+import torch
+
+from tests.gpu_common import rand_int8, randn
+from wgpkernels_b200 import build as builder
+
+
+@pytest.fixture(scope="module")
+def native():
+    builder.build()
+    from wgpkernels_b200.int8 import _calls
+    return _calls
+
+
+def test_takes_cuda_tensors_only(native):
+    x, w, s = torch.zeros(2, 256, dtype=torch.bfloat16), torch.zeros(8, 256, dtype=torch.int8), torch.ones(8)
+    tensors = (x, w, s, None, None, None, None, None)
+    assert native.linear(0, *tensors, 0, 0, 0.0, 1, 1, 148, 4096) is None
+    assert native.few(0, *tensors, 0, 0.0, 1, 148, 0, 0) is None
+    assert native.linear(0, [x], *tensors[1:], 0, 0, 0.0, 1, 1, 148, 4096) is None  # what is no tensor
+
+
+def test_wrong_arguments_are_errors(native):
+    with pytest.raises(TypeError):
+        native.linear(0)
+    with pytest.raises(TypeError):
+        native.few(0, None)
+    with pytest.raises(TypeError):
+        native.linear(0, *[None] * 8, "group", 0, 0.0, 1, 1, 148, 4096)
+
+
+class Marked(torch.Tensor):
+    pass
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,mode", [(1, "lines"), (12, "small"), (40, "exact"), (40, "block")])
+def test_other_forms_take_the_general_way(wq, m, mode, monkeypatch):
+    n, k = 264, 2048
+    x, w, s, b = randn((m, k), torch.float16, 1).cuda(), rand_int8((n, k), 2).cuda(), (torch.rand(n) * 0.01 + 0.001).cuda(), randn((n,), torch.float16, 3).cuda()
+    res = randn((m, n), torch.float16, 4).cuda()
+    wq.linear(x, w, s, b, mode=mode)  # (the tile variant is known from here on)
+    expected, added = wq.linear(x, w, s, b, mode=mode), wq.linear(x, w, s, b, mode=mode, residual=res)
+    taken = []
+    native = wq._native
+    monkeypatch.setattr(wq, "_native", type("Counted", (), {name: staticmethod(lambda *a, f=getattr(native, name): taken.append(f(*a)) or taken[-1]) for name in ("linear", "few")}))
+    assert torch.equal(wq.linear(torch.nn.Parameter(x, requires_grad=False), w, s, b, mode=mode), expected) and taken.pop() is not None
+    out = torch.empty_like(res)
+    assert wq.linear(x, w, s, b, mode=mode, residual=res, out=out) is out and torch.equal(out, added) and taken.pop() is out
+    general = wq.linear(x.as_subclass(Marked), w, s, b, mode=mode)
+    assert taken.pop() is None and torch.equal(general.as_subclass(torch.Tensor), expected)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        elsewhere = wq.linear(x, w, s, b, mode=mode)
+    side.synchronize()
+    assert torch.equal(elsewhere, expected)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = wq.linear(x, w, s, b, mode=mode)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(captured, expected)
+
+
+@pytest.mark.gpu
+def test_library_errors_are_raised(wq):
+    x, w, s = torch.zeros(12, 2048 + 8, dtype=torch.float16, device="cuda")[:, 4:2052], torch.zeros(8, 2048, dtype=torch.int8, device="cuda"), torch.ones(8, device="cuda")
+    with pytest.raises(RuntimeError):  # rows that are not 16-byte aligned
+        wq.linear(x, w, s, mode="small")

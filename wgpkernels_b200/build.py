@@ -2,7 +2,8 @@
 
     python -m wgpkernels_b200.build [--output PATH] [--verbose] [--jobs N] [--force]
 
-A second, tiny library, libwgp_int8_probe.so, is built beside it: the tensor-pipe issue-rate probe that only the benchmark loads.
+A second, tiny library, libwgp_int8_probe.so, is built beside it: the tensor-pipe issue-rate probe that only the benchmark loads.  And the native
+host side of the Python module, _calls.so, with the C++ compiler against the PyTorch at hand.
 
 One architecture only: the GEMM uses tcgen05 / tensor-memory instructions that exist on sm_100a alone, so there is no PTX fallback.
 The CUDA runtime is linked statically and only the C ABI is exported, so the library depends on the driver alone (the same properties
@@ -11,7 +12,9 @@ as the reference's build, wgpkernels/build.py:55-65 of WGPKernels).
 import argparse
 import os
 import re
+import shutil
 import subprocess
+import sysconfig
 import tempfile
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
@@ -50,6 +53,32 @@ def probe_library_file():
     return PACKAGE / "int8" / "libwgp_int8_probe.so"
 
 
+def calls_file():
+    return PACKAGE / "int8" / "_calls.so"
+
+
+def build_calls(nvcc="nvcc", verbose=False, force=False):
+    """Compiles the native host side of the Python module (a CPython extension) against the PyTorch that imports it."""
+    import torch
+    source, target, root = PACKAGE / "csrc" / "host_calls.cpp", calls_file(), Path(torch.__file__).resolve().parent
+    if not force and not _stale(target, [source]):
+        return target
+    toolkit = Path(shutil.which(nvcc) or "/usr/local/cuda/bin/nvcc").resolve().parents[1]
+    includes = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"], toolkit / "include"]
+    with tempfile.TemporaryDirectory(prefix="wgpkernels-b200-") as work:
+        built = Path(work) / target.name
+        done = subprocess.run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+                               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{path}" for path in includes], str(source), f"-L{root / 'lib'}",
+                               "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-o", str(built)], capture_output=True, text=True)
+        if verbose or done.returncode:
+            print(done.stdout + done.stderr)
+        if done.returncode:
+            raise RuntimeError(f"the C++ compiler failed on {source.name}")
+        target.write_bytes(built.read_bytes())
+    target.chmod(0o755)
+    return target
+
+
 def _stale(target, sources):
     if not target.exists():
         return True
@@ -61,6 +90,7 @@ def build(output=None, nvcc="nvcc", verbose=False, jobs=None, force=False, sourc
     """Compiles `sources` into the shared library `output` (default: the product library; the probe library is built with it)."""
     if output is None and sources is SOURCES:
         build(probe_library_file(), nvcc, verbose, jobs, force, PROBE_SOURCES)
+        build_calls(nvcc, verbose, force)
     target = Path(output or library_file()).resolve()
     csrc = PACKAGE / "csrc"
     inputs = [csrc / name for name in sources] + [csrc / name for name in HEADERS]
