@@ -488,3 +488,24 @@ def test_residual_through_the_staging_tiles(wq, shape, mode, staged, loaded):
         if n % 8 == 0:
             assert torch.equal(call(variant, residual=wide[:, 8:8 + n], out=torch.empty_like(res)), expected)
     assert wq.debug_status() == 0
+
+
+@pytest.mark.parametrize("mode,staged,one_tile", [("block", 10, 20), ("block+g", 12, 13)])
+@pytest.mark.parametrize("shape", [(12800, 520, 128), (9001, 1000, 128), (6000, 2312, 256)], ids=str)
+def test_edge_tiles_and_whole_tiles_of_one_cta(wq, shape, mode, staged, one_tile):
+    """Without a residual: tiles that N cuts off, written through one staging tile, and whole ones, written through two, on the same CTAs with a
+    block or two of K between them.  The bits of the kernel that has one staging tile a warp; the segments of one launch as well."""
+    m, n, k = shape
+    dtype = torch.bfloat16
+    _, a, _, sa, b, sb, bias, _, _ = operands(mode, m, n, k, dtype, 38, False)
+    a, sa, b, sb, bias = (t.cuda() for t in (a, sa, b, sb, bias))
+    expected = wq.gemm(a, None, sa, b, sb, bias, dtype, 0, one_tile)
+    for _ in range(5):
+        assert torch.equal(wq.gemm(a, None, sa, b, sb, bias, dtype, 0, staged), expected)
+    if mode == "block":
+        wq._plans[("block", m, 2 * n, k, a.device.index)] = (staged, 0, 0, 0)
+        outputs = [torch.empty_like(expected) for _ in range(2)]
+        wq.linear_prepared_segments(wq.Prepared("block", a, None, sa, dtype), [b, b], [sb, sb], [bias, bias], outputs)
+        assert all(torch.equal(out, expected) for out in outputs)
+        del wq._plans[("block", m, 2 * n, k, a.device.index)]
+    assert wq.debug_status() == 0

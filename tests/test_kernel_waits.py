@@ -46,6 +46,18 @@ def test_aborting_producers_wait_for_the_copies_they_issued(name):
     assert "await_issued_fills(bar_full, kStages" in code(name) and "mbar_try_wait(" not in code(name)
 
 
+def test_staging_tiles_are_written_again_only_behind_every_store():
+    """The tiles of one launch go out in two ways, through one staging tile of a warp or through one a chunk, so the number of stores behind a staging
+    tile's last reader is not known: a warp waits for all of them (a wait that lets some be pending lets one go on reading what is written again)."""
+    text = code("gemm_tc.cu")
+    waits = re.findall(r"cp\.async\.bulk\.wait_group\.read ([^;]+);", text)
+    assert len(waits) >= 3 and set(waits) == {"0"}
+    fast = text[text.index("auto emit_fast ="):text.index("if constexpr (S::kFold)", text.index("auto emit_fast ="))]
+    free = fast[fast.index("auto staging_free ="):fast.index("constexpr bool kAtOnce")]
+    assert re.findall(r"if \((.*)\) return;", free) == ["S::kStoreTiles > 1 && chunk > 0"]
+    assert fast.index("if constexpr (kAtOnce) staging_free();") < fast.index("stage_piece(g, packed)") and fast.rindex("staging_free();") < fast.rindex("stage_piece(")
+
+
 def test_warps_that_meet_at_a_named_barrier_agree_there():
     """The drain warps of the few-token kernel meet once per shared tile; a warp that gave up has to come there as well."""
     text = code("stream_tc.cu")

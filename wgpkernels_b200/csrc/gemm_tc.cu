@@ -687,10 +687,13 @@ gemm_i8_tc(const __grid_constant__ InputMaps in_maps, const __grid_constant__ We
             };
             auto emit_fast = [&](const float2* a, int chunk, const uint4* res, bool has_res) {
                 const int ct = part * kEpi + chunk * 32;  // first column of the chunk within the tile
-                // The TMA store that last read the staging tile must be done with it.  Of two tiles that is the store before last: over, so the outputs go
-                // there as they come (fewer registers); of one, it is awaited behind the arithmetic.
+                // The TMA store that last read the staging tile must be done with it.  With one tile that is awaited behind the arithmetic.  With a tile
+                // for each chunk the first chunk waits for ALL the stores of the tile before: long over, so the outputs go there as they come
+                // (fewer registers), and nothing is left to wait for at the chunks behind it.  (Which of those stores read which staging
+                // tile is not known: `emit`, at the right edge of N, sends every chunk through the first one.)
                 auto staging_free = [&]() {
-                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(S::kStoreTiles - 1) : "memory");
+                    if (S::kStoreTiles > 1 && chunk > 0) return;
+                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                     __syncwarp();
                 };
                 constexpr bool kAtOnce = S::kStoreTiles > 1;
