@@ -167,7 +167,8 @@ int wq8_stream_planes(const void* x, int64_t ldx, const int8_t* w, const float* 
  * rows of 2 K, gate | value --, 3 gelu): op(X) is rounded to X's type, as wq8_transform_rows does.  wq8_few_takes() says how a shape runs:
  *   1  one launch, no scratch: up to four tokens, the shapes of wq8_stream_planes whose digit planes fit beside the weights, not rms_norm (every CTA
  *      makes the planes for itself while its first weights are on their way); x 8-byte aligned, ldx a multiple of 4
- *   2  two launches: the other shapes that wq8_small runs on tcgen05, up to 32 tokens; slots and counters as wq8_small_workspace() reports; x and
+ *   2  two launches: the other shapes that wq8_small runs on tcgen05, up to 32 tokens; slots and counters of the sizes wq8_small_workspace() reports, both this
+ *      call's own until it has run (the counters are cleared by the call itself: no need to hand in zeros); x and
  *      act_weight 16-byte aligned, ldx a multiple of 8
  *   0  not at all (-2 from wq8_few).  w 16-byte aligned.  No counterpart in the reference (which launches the input operation and the product
  * separately). */

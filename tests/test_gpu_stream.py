@@ -185,6 +185,42 @@ def test_input_operation_and_stream_in_one_launch(wq, m, shape, act, dtype):
     assert wq.debug_status() == 0
 
 
+@pytest.mark.parametrize("form", ["linear", "prepared"])
+@pytest.mark.parametrize("m,act", [(1, "rms_norm"), (3, None), (16, "gelu")], ids=str)
+def test_calls_on_several_streams_count_their_own_pieces(wq, m, act, form):
+    """Tiles that several CTAs share, on streams that nothing orders and that prepare_stream() has not seen: the bits of a call alone.  The device's
+    shared counters, whatever they hold, are no part of it."""
+    n, k = 520, 6144
+    _, w, sw, bias, _, _ = case(m, n, k, torch.float16, 161, False)
+    xs = [randn((m, k), torch.float16, 162 + i).cuda() for i in range(4)]
+    gw, gsw, gbias = cuda(w, sw, bias)
+    assert wq._require().wq8_few_takes(m, n, k, wq.ACTS[act], 148) == 2
+
+    def call(x):
+        if form == "linear":
+            return wq.linear(x, gw, gsw, gbias, mode="small", act=act, eps=1e-6)
+        return wq.linear_prepared(wq.prepare(x, 0, "small", act, None, 1e-6), gw, gsw, gbias)
+
+    alone = [call(x) for x in xs]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in xs]
+    shared = wq._counters[0].clone()
+    wq._counters[0].fill_(3)
+    torch.cuda.synchronize()
+    try:
+        for _ in range(20):
+            together = []
+            for stream, x in zip(streams, xs):
+                with torch.cuda.stream(stream):
+                    together.append(call(x))
+            torch.cuda.synchronize()
+            assert all(torch.equal(a, b) for a, b in zip(alone, together))
+        assert bool((wq._counters[0] == 3).all())
+    finally:
+        wq._counters[0].copy_(shared)
+    assert wq.debug_status() == 0
+
+
 def test_how_the_shapes_run(wq):
     takes = wq._require().wq8_few_takes
     assert [takes(m, 4096, 4096, 0, 148) for m in (1, 2, 3, 4, 5, 32, 33)] == [1, 1, 1, 1, 2, 2, 0]

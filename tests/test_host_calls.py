@@ -1,9 +1,12 @@
 """The native host side of the two whole-linear library calls: which calls it takes, and that the others go the general way with the same bits."""
+from types import SimpleNamespace
+
 import pytest
 import torch
 
 from tests.gpu_common import rand_int8, randn
 from wgpkernels_b200 import build as builder
+from wgpkernels_b200 import int8
 
 
 @pytest.fixture(scope="module")
@@ -32,6 +35,21 @@ def test_wrong_arguments_are_errors(native):
 
 class Marked(torch.Tensor):
     pass
+
+
+def test_tile_counters_lie_in_the_calls_own_scratch(monkeypatch):
+    """What streams would share is no part of a few-token call: its scratch holds its counters, behind the partial sums."""
+    def workspace(m, n, k, sms, sizes):
+        sizes[0], sizes[1] = 1024, 64
+
+    calls = []
+    library = SimpleNamespace(wq8_few_takes=lambda *shape: 2, wq8_small_workspace=workspace)
+    for name, value in (("_lib", library), ("_sms", {None: 148}), ("_few_shapes", {}), ("_native", SimpleNamespace(few=lambda *a: calls.append(a[-2:]) or "done")),
+                        ("_stream", None), ("_zeroed_counters", None)):
+        monkeypatch.setattr(int8, name, value)
+    x, w, s = torch.zeros(2, 256, dtype=torch.bfloat16), torch.zeros(8, 256, dtype=torch.int8), torch.ones(8)
+    assert int8._with_input_operation(x, w, s, None, 0, "rms_norm", None, 1e-6, None, None, None) == "done"
+    assert calls == [(1024 + 64, 1024)]
 
 
 @pytest.mark.gpu

@@ -278,7 +278,7 @@ int gemm_few_rows_launch(const int8_t* a, const int8_t* a_lo, const float* sa, c
                          const void* rscale, void* y, int64_t ld_y, int64_t ld_residual, int m, int n, int k, bool is_bf16, int sms, cudaStream_t stream);
 int gemm_rows_status_take();
 // stream_tc.cu: the few-token linear on tcgen05 (digit planes): scratch bytes of a shape (0: not this kernel's shape; *counter_bytes: its
-// tile counters), the launch (act: input operation of x; workspace and zeroed counters of those sizes), and its status word
+// tile counters), the launch (act: input operation of x; workspace and counters of those sizes, this call's own), and its status word
 int64_t stream_tc_workspace(int m, int n, int k, int sms, int64_t* counter_bytes);
 int stream_tc_launch(const void* x, int64_t ldx, int act, const void* act_weight, float eps, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale, void* y, int m,
                      int n, int k, int dtype, int sms, void* workspace, int* counters, cudaStream_t stream);

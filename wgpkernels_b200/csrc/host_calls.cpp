@@ -5,7 +5,7 @@
 // class, strides, types) comes back as None and takes the general way.
 //
 //   linear(address, x, weight, scale, bias, residual, residual_scale, out, act_weight, group, act, eps, path, variant, sms, scratch bytes)
-//   few(address, x, weight, scale, bias, residual, residual_scale, out, act_weight, act, eps, form, sms, scratch bytes, counters)
+//   few(address, x, weight, scale, bias, residual, residual_scale, out, act_weight, act, eps, form, sms, scratch bytes, where in them the tile counters lie)
 //
 // both return the output, None, or the library's error code as an int.  Built against the PyTorch that runs it, without CUDA code of its own.
 #define PY_SSIZE_T_CLEAN
@@ -120,7 +120,7 @@ PyObject* few(PyObject*, PyObject* const* a, Py_ssize_t count) {
     const int act = integer(a[9]), form = integer(a[11]), sms = integer(a[12]);
     const auto eps = float(PyFloat_AsDouble(a[10]));
     const int64_t bytes = PyLong_AsLongLong(a[13]);
-    void* counters = PyLong_AsVoidPtr(a[14]);
+    const int64_t counters = PyLong_AsLongLong(a[14]);
     if (PyErr_Occurred()) return nullptr;
     Operands o;
     if (!take(a + 1, act, o)) Py_RETURN_NONE;
@@ -131,9 +131,10 @@ PyObject* few(PyObject*, PyObject* const* a, Py_ssize_t count) {
     allocate_output(o);
     const at::Tensor scratch = bytes ? scratch_of(o, bytes) : at::Tensor();
     void *y = o.out.data_ptr(), *memory = bytes ? scratch.data_ptr() : nullptr, *stream = stream_of(o);
+    void* tile_counters = bytes ? static_cast<char*>(memory) + counters : nullptr;  // of this call alone: other streams' calls count their own
     return result(o, without_gil([&] {
                       return call(x, o.x.stride(0), w, static_cast<const float*>(o.scale), o.bias, o.residual, o.rscale, y, int(o.m), int(o.n), int(o.k), o.dtype, act,
-                                  o.act_weight, eps, sms, memory, counters, stream);
+                                  o.act_weight, eps, sms, memory, tile_counters, stream);
                   }));
     END_HANDLE_TH_ERRORS
 }

@@ -16,7 +16,8 @@
 // Work is spread stream-K style: the (channel tile, K block) pairs are numbered linearly and every CTA takes one contiguous share of
 // them, so all SMs stream for the same time whatever N and K are.  A tile whose K range is shared by several CTAs is finished by the
 // last one to arrive (a counter per tile): every piece is written to a slot of the caller's scratch, and the last arriver adds the
-// pieces in CTA order -- a fixed order, so the result does not depend on timing.  Counters are zero on entry and left zero.
+// pieces in CTA order -- a fixed order, so the result does not depend on timing.  The counters are the call's own: the digit split in front clears
+// them, so calls on different streams do not count each other's pieces.
 //
 // Every wait is bounded (tc_ptx.cuh): a wait that gives up records a code in the status word of the streaming kernels, raises the
 // CTA's abort flag, and the CTA leaves through the common exit with tensor memory released.
@@ -55,7 +56,7 @@ template <int TB> struct TcShape {
 // tokens x 14336, SwiGLU, 2.3 + 2.4 us -> 2.5.
 template <class T, int TB, int ACT>
 __global__ void __launch_bounds__(kRowThreads) split_digits(const T* x, int64_t ldx, const T* act_weight, float eps, int8_t* __restrict__ digits,
-                                                            float* __restrict__ scales, int m, int k) {
+                                                            float* __restrict__ scales, int m, int k, int* counters, int tiles) {
     __shared__ float slots[9];
     // This kernel may have started under the tail of the one that produced x.  Once that has finished, the stream kernel that follows may
     // start (its set-up and its first weight loads do not depend on the digits; the weights themselves may come from the kernel waited for
@@ -63,6 +64,9 @@ __global__ void __launch_bounds__(kRowThreads) split_digits(const T* x, int64_t 
     dependency_wait();
     dependents_may_start();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, token = blockIdx.x;
+    // the tile counters of the stream kernel, which belong to this call: whatever they held, it finds zeros
+    if (blockIdx.x == 0 && blockIdx.y == 0)
+        for (int i = threadIdx.x; i < tiles; i += kRowThreads) counters[i] = 0;
     const T* row = x + int64_t(token) * ldx;
     const bool used = token < m;
     auto load = [&](const T* p, float* v, bool valid) {
@@ -144,7 +148,7 @@ struct TcParams {
     const void* rscale;
     void* y;
     float* slots;          // 2 pieces of kPieceFloats per CTA
-    int* counters;         // one per tile, zero on entry, left zero
+    int* counters;         // one per tile, cleared by the split, left zero
     int m, n, k, tiles, kblocks;
 };
 
@@ -463,7 +467,8 @@ static int launch_tc_shape(const T* x, int64_t ldx, int act, const T* act_weight
     if (act == kActSwiglu) splitter = split_digits<T, TB, kActSwiglu>;
     if (act == kActGelu) splitter = split_digits<T, TB, kActGelu>;
     const cudaError_t split =
-        launch_after_previous(splitter, grid, dim3(kRowThreads), size_t(0), stream, x, ldx, act_weight, eps, digits, scales, m, k);
+        launch_after_previous(splitter, grid, dim3(kRowThreads), size_t(0), stream, x, ldx, act_weight, eps, digits, scales, m, k, counters,
+                              (n + kTcChannels - 1) / kTcChannels);
     if (split != cudaSuccess) return int(split);
     TcParams p{scales, sw, bias, residual, rscale, y, slots, counters, m, n, k, (n + kTcChannels - 1) / kTcChannels, runs};
     // behind the split: the stream kernel's set-up and first weight loads run under the split's tail
@@ -471,7 +476,8 @@ static int launch_tc_shape(const T* x, int64_t ldx, int act, const T* act_weight
     return int(launched != cudaSuccess ? launched : cudaGetLastError());
 }
 
-// x (m, K) in T (SwiGLU: (m, 2 K)); workspace: digits, then scales, then slots (plan sizes, each rounded up to 256 bytes); counters zeroed.
+// x (m, K) in T (SwiGLU: (m, 2 K)); workspace: digits, then scales, then slots (plan sizes, each rounded up to 256 bytes); counters: any memory of this
+// call's own (the split clears them).
 template <class T>
 static int launch_tc(const void* x, int64_t ldx, int act, const void* act_weight, float eps, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale, void* y, int m,
                      int n, int k, const TcPlan& plan, void* workspace, int* counters, cudaStream_t stream) {
