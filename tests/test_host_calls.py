@@ -52,6 +52,26 @@ def test_tile_counters_lie_in_the_calls_own_scratch(monkeypatch):
     assert calls == [(1024 + 64, 1024)]
 
 
+@pytest.mark.parametrize("m,mode,taken", [(1, "lines", True), (4, "lines", True), (5, "lines", False), (32, "lines", False), (4, "small", True), (32, "small", True),
+                                           (33, "small", False)])
+def test_which_token_counts_take_the_few_token_call(m, mode, taken, monkeypatch):
+    """'lines' is for one to four tokens: with more it is refused by the general way, not run as something else."""
+    for name, value in (("_lib", SimpleNamespace(wq8_few_takes=lambda *shape: 1)), ("_sms", {None: 148}), ("_few_shapes", {}),
+                        ("_native", SimpleNamespace(few=lambda *a: "few tokens")), ("linear_prepared", lambda *a: "general")):
+        monkeypatch.setattr(int8, name, value)
+    x, w, s = torch.zeros(m, 2048, dtype=torch.bfloat16), torch.zeros(8, 2048, dtype=torch.int8), torch.ones(8)
+    assert int8.linear(x, w, s, mode=mode) == ("few tokens" if taken else "general")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [5, 32])
+def test_lines_with_more_than_four_tokens_is_an_error(wq, m):
+    x, w, s = randn((m, 2048), torch.float16, 1).cuda(), rand_int8((8, 2048), 2).cuda(), torch.ones(8, device="cuda")
+    for act in (None, "rms_norm"):
+        with pytest.raises(RuntimeError, match="-2"):
+            wq.linear(x, w, s, mode="lines", act=act, eps=1e-6)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("m,mode", [(1, "lines"), (12, "small"), (40, "exact"), (40, "block")])
 def test_other_forms_take_the_general_way(wq, m, mode, monkeypatch):
