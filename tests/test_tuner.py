@@ -1,6 +1,8 @@
 """Host-side policy of the INT8 module without a GPU: buckets, the on-disk cache, the path rule (fastest full-precision path unless
 it costs more than 10% over 'block'), the untimed fallbacks used during CUDA graph capture, and the loud failure without a library."""
 import json
+import threading
+from types import SimpleNamespace
 
 import pytest
 import torch
@@ -134,6 +136,26 @@ def test_tile_tuner_picks_the_fastest_candidate(tuner):
     assert tuner._tuned_config(100, 96, 256, a.device, "exact", lambda option: None) == ((1, 0), True)
     assert len(tuner.calls) == before
     assert set(tuner._MODES[v] for mode, candidates in tuner._CANDIDATES.items() for v, _ in candidates if tuner._MODES[v] != mode) == set()
+
+
+def test_sizes_of_calls_in_several_threads(tuner, monkeypatch):
+    """A workspace query runs without the interpreter's lock: another thread may make its own between a query's end and the reading of its answer."""
+    device, meanwhile = torch.device("cuda", 0), []
+
+    def query(m, n, k, *rest):
+        sizes = rest[-1]
+        sizes[0], sizes[1] = 1000 * m, m
+        if meanwhile:
+            thread = threading.Thread(target=meanwhile.pop())
+            thread.start()
+            thread.join()
+
+    monkeypatch.setattr(tuner, "_lib", SimpleNamespace(wq8_gemm_workspace=query, wq8_small_workspace=query, wq8_few_takes=lambda *shape: 2))
+    monkeypatch.setattr(tuner, "_sms", {0: 148})
+    meanwhile.append(lambda: tuner._few_shape(3, 96, 256, None, device))
+    assert tuner._few_shape(20, 96, 256, None, device) == (2, 20020, 20000)
+    meanwhile.append(lambda: tuner._plan(64, 96, 256, device, "exact+g", None))
+    assert tuner._plan(100, 96, 256, device, "exact+g", None) == (14, 0, 100000, 100) and tuner._plans[("exact+g", 64, 96, 256, 0)][2:] == (64000, 64)
 
 
 def test_no_library_no_result(monkeypatch):
