@@ -56,6 +56,9 @@ def test_cache_round_trip_and_version(tuner):
     tuner._TUNING_PATH.write_text(json.dumps({"version": tuner._TUNING_VERSION + 1, "configs": {"key": [11, 0]}}))
     tuner._tuned = None
     assert tuner._cache() == {}  # another version's tile ids are never read
+    tuner._TUNING_PATH.write_text(json.dumps({"version": 3, "configs": {"path|4x96x256|g0|Fake B200": "small"}}))
+    tuner._tuned = None
+    assert tuner._cache() == {}  # nor what was timed before the kernels for few tokens and few rows
     tuner._TUNING_PATH.write_text("{not json")
     tuner._tuned = None
     assert tuner._cache() == {}
