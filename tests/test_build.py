@@ -1,4 +1,4 @@
-"""The build's check of ptxas' report (no GPU)."""
+"""The build's check of ptxas' report, and how it puts a new library in place (no GPU)."""
 from wgpkernels_b200 import build as builder
 
 
@@ -15,3 +15,14 @@ def test_spills_around_tensor_memory_loads_are_refused():
     assert builder.spills(fine) == []
     bad = fine + report(row, 8, 4) + report(block, 16, 4) + report(eight_warps, 8, 8) + report(few, 4, 4)
     assert builder.spills(bad) == [(row, 8, 4), (block, 16, 4), (eight_warps, 8, 8), (few, 4, 4)]
+
+
+def test_a_new_file_takes_the_old_ones_place(tmp_path):
+    """Not its bytes: a process that has the old library mapped goes on with it."""
+    target, built = tmp_path / "library.so", tmp_path / "new"
+    target.write_bytes(b"old")
+    built.write_bytes(b"new and longer")
+    with open(target, "rb") as mapped:
+        builder._install(built, target)
+        assert mapped.read() == b"old" and target.read_bytes() == b"new and longer"
+    assert sorted(path.name for path in tmp_path.iterdir()) == ["library.so", "new"]

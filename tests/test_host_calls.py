@@ -16,6 +16,25 @@ def native():
     return _calls
 
 
+def test_is_bound_to_the_pytorch_it_was_built_for(native, tmp_path, monkeypatch):
+    """The file says what it was compiled against; with another PyTorch or Python it is not used, and a build makes it anew."""
+    assert native.BUILT_FOR == builder.built_for() and torch.__version__ in native.BUILT_FOR
+    monkeypatch.setattr(int8, "built_for", lambda: "another PyTorch")
+    with pytest.raises(RuntimeError, match="another PyTorch; rebuild it"):
+        int8._native_calls()
+    current = builder.calls_file()
+    copy = tmp_path / "_calls.so"
+    copy.write_bytes(current.read_bytes())
+    monkeypatch.setattr(builder, "calls_file", lambda: copy)
+    compiled = []
+    monkeypatch.setattr(builder.subprocess, "run", lambda command, **kw: compiled.append(command) or SimpleNamespace(returncode=1, stdout="", stderr=""))
+    assert builder.build_calls() == copy and not compiled
+    monkeypatch.setattr(builder, "built_for", lambda: "torch of tomorrow")
+    with pytest.raises(RuntimeError, match="compiler failed"):
+        builder.build_calls()
+    assert any('-DWQ_BUILT_FOR="torch of tomorrow"' in argument for argument in compiled[0])
+
+
 def test_takes_cuda_tensors_only(native):
     x, w, s = torch.zeros(2, 256, dtype=torch.bfloat16), torch.zeros(8, 256, dtype=torch.int8), torch.ones(8)
     tensors = (x, w, s, None, None, None, None, None)

@@ -14,6 +14,7 @@ import os
 import re
 import shutil
 import subprocess
+import sys
 import sysconfig
 import tempfile
 from concurrent.futures import ThreadPoolExecutor
@@ -57,26 +58,41 @@ def calls_file():
     return PACKAGE / "int8" / "_calls.so"
 
 
+def built_for():
+    """The PyTorch and the Python at hand, as the native host side names those it was compiled against: it reads tensors through PyTorch's inline
+    functions, so with others it may import and read wrong offsets."""
+    import torch
+    return f"torch {torch.__version__} {torch.version.git_version}, {sys.implementation.cache_tag}, C++11 ABI {int(torch._C._GLIBCXX_USE_CXX11_ABI)}"
+
+
 def build_calls(nvcc="nvcc", verbose=False, force=False):
     """Compiles the native host side of the Python module (a CPython extension) against the PyTorch that imports it."""
     import torch
     source, target, root = PACKAGE / "csrc" / "host_calls.cpp", calls_file(), Path(torch.__file__).resolve().parent
-    if not force and not _stale(target, [source]):
+    identity = built_for()
+    if not force and not _stale(target, [source]) and identity.encode() in target.read_bytes():
         return target
     toolkit = Path(shutil.which(nvcc) or "/usr/local/cuda/bin/nvcc").resolve().parents[1]
     includes = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"], toolkit / "include"]
     with tempfile.TemporaryDirectory(prefix="wgpkernels-b200-") as work:
         built = Path(work) / target.name
         done = subprocess.run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-                               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{path}" for path in includes], str(source), f"-L{root / 'lib'}",
+                               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DWQ_BUILT_FOR="{identity}"', *[f"-I{path}" for path in includes], str(source), f"-L{root / 'lib'}",
                                "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-o", str(built)], capture_output=True, text=True)
         if verbose or done.returncode:
             print(done.stdout + done.stderr)
         if done.returncode:
             raise RuntimeError(f"the C++ compiler failed on {source.name}")
-        target.write_bytes(built.read_bytes())
-    target.chmod(0o755)
+        _install(built, target)
     return target
+
+
+def _install(built, target):
+    """Puts a new file in the old one's place: a process that has the old one mapped keeps it whole."""
+    beside = target.with_name(f"{target.stem}.{os.getpid()}.so")
+    shutil.copyfile(built, beside)
+    beside.chmod(0o755)
+    os.replace(beside, target)
 
 
 def _stale(target, sources):
@@ -115,7 +131,7 @@ def build(output=None, nvcc="nvcc", verbose=False, jobs=None, force=False, sourc
         built = Path(work) / target.name
         subprocess.run([nvcc, "-shared", *ARCH_FLAGS, "--cudart", "static", "-Xcompiler", "-fPIC,-fvisibility=hidden",
                         *map(str, objects), "-o", str(built)], check=True)
-        target.write_bytes(built.read_bytes())
+        _install(built, target)
     return target
 
 

@@ -7,7 +7,8 @@
 //   linear(address, x, weight, scale, bias, residual, residual_scale, out, act_weight, group, act, eps, path, variant, sms, scratch bytes)
 //   few(address, x, weight, scale, bias, residual, residual_scale, out, act_weight, act, eps, form, sms, scratch bytes, where in them the tile counters lie)
 //
-// both return the output, None, or the library's error code as an int.  Built against the PyTorch that runs it, without CUDA code of its own.
+// both return the output, None, or the library's error code as an int.  Built against the PyTorch that runs it
+// (BUILT_FOR names it; another one may lay tensors out otherwise), without CUDA code of its own.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -146,4 +147,15 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_calls", "Native host side of wq8_
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__calls() { return PyModule_Create(&module); }
+#ifndef WQ_BUILT_FOR
+#error "the build passes the PyTorch and the Python that this is compiled against"
+#endif
+
+PyMODINIT_FUNC PyInit__calls() {
+    PyObject* made = PyModule_Create(&module);
+    if (made && PyModule_AddStringConstant(made, "BUILT_FOR", WQ_BUILT_FOR) < 0) {
+        Py_DECREF(made);
+        return nullptr;
+    }
+    return made;
+}
