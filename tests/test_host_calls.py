@@ -4,7 +4,7 @@ from types import SimpleNamespace
 import pytest
 import torch
 
-from tests.gpu_common import rand_int8, randn
+from tests.gpu_common import rand_int8, randn, rel
 from wgpkernels_b200 import build as builder
 from wgpkernels_b200 import int8
 
@@ -33,6 +33,30 @@ def test_is_bound_to_the_pytorch_it_was_built_for(native, tmp_path, monkeypatch)
     with pytest.raises(RuntimeError, match="compiler failed"):
         builder.build_calls()
     assert any('-DWQ_BUILT_FOR="torch of tomorrow"' in argument for argument in compiled[0])
+
+
+def test_loads_without_the_native_side(native, monkeypatch):
+    """The library is what computes: without its native callers linear() makes its calls one by one."""
+    def missing():
+        raise RuntimeError("the native host side is missing")
+
+    for name in ("_lib", "_native", "_linear_address", "_few_address", "_weight_groups"):
+        monkeypatch.setattr(int8, name, getattr(int8, name))
+    monkeypatch.setattr(int8, "_native_calls", missing)
+    with pytest.warns(RuntimeWarning, match="is missing"):
+        library = int8.load_library(builder.build())
+    assert int8._lib is library and int8._native is None
+    monkeypatch.setattr(int8, "_plans", {("exact", 40, 8, 256, None): (1, 0, 0, 0)})
+    x, w, s = torch.zeros(40, 256, dtype=torch.bfloat16), torch.zeros(8, 256, dtype=torch.int8), torch.ones(8)
+    assert int8._one_call(x, w, s, None, 0, "exact", None, None, 0.0, None, None, None) is None
+    assert int8._with_input_operation(x[:4], w, s, None, 0, None, None, 0.0, None, None, None) is None
+
+
+def test_a_build_elsewhere_makes_it_as_well(tmp_path, monkeypatch):
+    made = []
+    monkeypatch.setattr(builder, "build_calls", lambda *a, **kw: made.append("calls"))
+    monkeypatch.setattr(builder, "_stale", lambda target, sources: False)
+    assert builder.build(tmp_path / "libwgp_int8.so") == (tmp_path / "libwgp_int8.so").resolve() and made == ["calls"]
 
 
 def test_takes_cuda_tensors_only(native):
@@ -119,6 +143,22 @@ def test_other_forms_take_the_general_way(wq, m, mode, monkeypatch):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(captured, expected)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("act", [None, "rms_norm"])
+@pytest.mark.parametrize("m,mode", [(1, "lines"), (12, "small"), (40, "exact"), (40, "block"), (300, "row")])
+def test_the_calls_one_by_one(wq, m, mode, act, monkeypatch):
+    """Without the native side: the same bits, but for one to four tokens behind rms_norm, whose sums are formed in another order."""
+    n, k = 264, 2048
+    x, w, s = randn((m, k), torch.float16, 1).cuda(), rand_int8((n, k), 2).cuda(), (torch.rand(n) * 0.01 + 0.001).cuda()
+    res = randn((m, n), torch.float16, 4).cuda()
+    call = lambda: wq.linear(x, w, s, None, mode=mode, act=act, eps=1e-6, residual=res)
+    call()
+    expected = call()
+    monkeypatch.setattr(wq, "_native", None)
+    assert rel(call(), expected) < 1e-4 if (m, act) == (1, "rms_norm") else torch.equal(call(), expected)
+    assert wq.debug_status() == 0
 
 
 @pytest.mark.gpu

@@ -104,9 +104,10 @@ def _stale(target, sources):
 
 def build(output=None, nvcc="nvcc", verbose=False, jobs=None, force=False, sources=SOURCES):
     """Compiles `sources` into the shared library `output` (default: the product library; the probe library is built with it)."""
-    if output is None and sources is SOURCES:
-        build(probe_library_file(), nvcc, verbose, jobs, force, PROBE_SOURCES)
-        build_calls(nvcc, verbose, force)
+    if sources is SOURCES:
+        build_calls(nvcc, verbose, force)  # (whichever library the module is to load, these lie beside the module)
+        if output is None:
+            build(probe_library_file(), nvcc, verbose, jobs, force, PROBE_SOURCES)
     target = Path(output or library_file()).resolve()
     csrc = PACKAGE / "csrc"
     inputs = [csrc / name for name in sources] + [csrc / name for name in HEADERS]
