@@ -52,6 +52,22 @@ def test_loads_without_the_native_side(native, monkeypatch):
     assert int8._with_input_operation(x[:4], w, s, None, 0, None, None, 0.0, None, None, None) is None
 
 
+def test_scratch_is_that_of_the_variant_and_library_in_use(native, monkeypatch):
+    """wq8_linear is not told how large its scratch is: a size kept from another tile variant, or another library, must not be passed."""
+    sizes = []
+    for name, value in (("_native", SimpleNamespace(linear=lambda *a: sizes.append(a[-1]) or "done")), ("_sms", {None: 148}), ("_plans", {}), ("_scratch_sizes", {}),
+                        ("_few_shapes", {"a shape": (1, 0, 0)}), ("_linear_address", 0), ("_few_address", 0), ("_weight_groups", False),
+                        ("_lib", SimpleNamespace(wq8_linear_scratch=lambda m, n, k, path, variant, sms: 1000 * variant))):
+        monkeypatch.setattr(int8, name, value)
+    x, w, s = torch.zeros(40, 256, dtype=torch.bfloat16), torch.zeros(8, 256, dtype=torch.int8), torch.ones(8)
+    for variant in (10, 20, 10):
+        int8._plans["block", 40, 8, 256, None] = (variant, 0, 0, 0)
+        assert int8._one_call(x, w, s, None, 0, "block", None, None, 0.0, None, None, None) == "done"
+    assert sizes == [10000, 20000, 10000]
+    int8.load_library(builder.build())
+    assert not int8._plans and not int8._scratch_sizes and not int8._few_shapes
+
+
 def test_a_build_elsewhere_makes_it_as_well(tmp_path, monkeypatch):
     made = []
     monkeypatch.setattr(builder, "build_calls", lambda *a, **kw: made.append("calls"))
