@@ -46,6 +46,39 @@ def test_aborting_producers_wait_for_the_copies_they_issued(name):
     assert "await_issued_fills(bar_full, kStages" in code(name) and "mbar_try_wait(" not in code(name)
 
 
+@pytest.mark.parametrize("name,wait,count", [("gemm_rows.cu", "rows_wait", 3), ("stream_few.cu", "few_wait", 3)])
+def test_waits_vote_at_the_call(name, wait, count):
+    text = code(name)
+    waits = [m for m in re.finditer(rf"(?<!\w){wait}\((?!uint32_t bar)", text)]
+    assert len(waits) == count and all(text[:m.start()].endswith("whole_warp(") for m in waits) and "mbar_try_wait(" not in text
+
+
+def test_every_thread_comes_to_the_clusters_barriers():
+    """Up to 128 rows: the CTAs of a cluster write into each other's shared memory between two barriers, which a CTA that gave up comes to as well,
+    with none of its copies in flight."""
+    text = code("gemm_rows.cu")
+    body = text[text.index("gemm_few_rows(const __grid_constant__"):text.index("bool make_swizzled_byte_map")]
+    meetings = [m.start() for m in re.finditer(r"__syncwarp\(\);\s*cluster_sync\(\);", body)]
+    assert len(meetings) == 2 == body.count("cluster_sync()")
+    assert not re.search(r"\breturn\b", body[:meetings[1]])
+    producer = body[body.index("if (warp == 0 && ok)"):body.index("else if (warp == 1 && ok)")]
+    assert re.search(r"[;}]\s*await_issued_fills\(bar_full, p\.stages, fills\);\s*\}\s*$", producer) and "return" not in producer
+    exchange = body.index("st.shared::cluster")
+    assert meetings[0] < exchange < meetings[1] and "if (warp >= 4 && complete)" in body[meetings[0]:exchange]
+
+
+def test_warps_of_one_launch_few_tokens_meet_whatever_became_of_their_waits():
+    """Two warps share a ring, sixteen the digits: a warp that gave up comes to every named barrier that the others wait at, and the one that requests
+    waits for its copies."""
+    text = code("stream_few.cu")
+    start = text.index("for (; segment < segments; segment += kFewPairs)")
+    loop = text[start:text.index("        segment -= segments;", start)]
+    pair_barrier = loop.index('asm volatile("bar.sync %0, 64;"')
+    assert loop[:pair_barrier].count("{") == loop[:pair_barrier].count("}") + 1  # in the loop itself, under no condition
+    assert not re.search(r"\b(break|continue|return)\b", loop)
+    assert 'if (item == 0 && segments % kFewPairs) asm volatile("bar.sync 1, %0;"' in text and "if (!ok && part == 0) await_issued_fills(bars, stages, fills);" in text
+
+
 def test_staging_tiles_are_written_again_only_behind_every_store():
     """The tiles of one launch go out in two ways, through one staging tile of a warp or through one a chunk, so the number of stores behind a staging
     tile's last reader is not known: a warp waits for all of them (a wait that lets some be pending lets one go on reading what is written again)."""

@@ -102,7 +102,9 @@ gemm_few_rows(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             }
             if (++stage == p.stages) stage = 0;
         }
-        if (!ok) await_issued_fills(bar_full, p.stages, fills);
+        // Whatever became of the waits, this one's or the issuer's: no copy is in flight when the stages become the place of the sums, or when the CTA
+        // leaves.  (The issuer waits for the same copies.)
+        await_issued_fills(bar_full, p.stages, fills);
     } else if (warp == 1 && ok) {
         // ---------------- MMA issuer ----------------
         const bool leader = elect_one();
