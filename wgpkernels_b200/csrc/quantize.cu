@@ -621,11 +621,15 @@ __global__ void __launch_bounds__(256) rotate_groups(const T* __restrict__ x, T*
 }
 
 // ---- host dispatch ----------------------------------------------------------------------------------------------------
-static int persistent_ctas(int64_t warps_of_work) {
+static int device_sm_count() {
     int device = 0, sms = 148;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const int64_t ctas = (warps_of_work + 7) / 8, cap = int64_t(sms) * 8;  // 8 CTAs of 256 threads fill an SM
+    return sms;
+}
+
+static int persistent_ctas(int64_t warps_of_work) {
+    const int64_t ctas = (warps_of_work + 7) / 8, cap = int64_t(device_sm_count()) * 8;  // 8 CTAs of 256 threads fill an SM
     return int(ctas < cap ? (ctas < 1 ? 1 : ctas) : cap);
 }
 
@@ -646,7 +650,7 @@ static int launch_blocks(const void* x, int8_t* q, float* scale, int m, int k, i
             // Four chunks a warp want enough warps: 20 an SM (BF16, 5888 values a row, one chunk a warp with tanhf and this, us: 256 rows 4.0
             // and 4.5, 512 5.9 and 5.7, 1560 14.0 and 10.9).
             const int64_t groups = (chunks + kGeluChunks - 1) / kGeluChunks;
-            if (m * groups >= 3000) {
+            if (m * groups >= 20 * device_sm_count()) {
                 const int64_t most = (int64_t(1) << 30) / groups;
                 for (int64_t row0 = 0; row0 < m; row0 += most) {
                     const uint32_t items = uint32_t((m - row0 < most ? m - row0 : most) * groups);
@@ -704,12 +708,16 @@ static int launch_rows(const void* x, int8_t* hi, int8_t* lo, float* scale, int 
             else quantize_rows_rotated<T, GROUP, HILO, 4><<<m, threads, 0, stream>>>(src, hi, lo, scale, k, ldx, shift);
             return int(cudaGetLastError());
         }
+    } else {
+        auto kernel = quantize_rows<T, GROUP, HILO, ACT, 0>;
+        if (k <= 2048) kernel = quantize_rows<T, GROUP, HILO, ACT, 1>;
+        else if (k <= 4096) kernel = quantize_rows<T, GROUP, HILO, ACT, 2>;
+        else if (k <= 8192) kernel = quantize_rows<T, GROUP, HILO, ACT, 4>;
+        else if (k <= 16384) kernel = quantize_rows<T, GROUP, HILO, ACT, 8>;
+        kernel<<<m, kRowThreads, 0, stream>>>(src, hi, lo, scale, k, ldx, aw, eps, shift);
+        return int(cudaGetLastError());
     }
-    if (k <= 2048) quantize_rows<T, GROUP, HILO, ACT, 1><<<m, kRowThreads, 0, stream>>>(src, hi, lo, scale, k, ldx, aw, eps, shift);
-    else if (k <= 4096) quantize_rows<T, GROUP, HILO, ACT, 2><<<m, kRowThreads, 0, stream>>>(src, hi, lo, scale, k, ldx, aw, eps, shift);
-    else if (k <= 8192) quantize_rows<T, GROUP, HILO, ACT, 4><<<m, kRowThreads, 0, stream>>>(src, hi, lo, scale, k, ldx, aw, eps, shift);
-    else if (k <= 16384) quantize_rows<T, GROUP, HILO, ACT, 8><<<m, kRowThreads, 0, stream>>>(src, hi, lo, scale, k, ldx, aw, eps, shift);
-    else quantize_rows<T, GROUP, HILO, ACT, 0><<<m, kRowThreads, 0, stream>>>(src, hi, lo, scale, k, ldx, aw, eps, shift);
+    quantize_rows<T, GROUP, HILO, ACT, 0><<<m, kRowThreads, 0, stream>>>(src, hi, lo, scale, k, ldx, aw, eps, shift);  // rotated rows of more than 16384 values
     return int(cudaGetLastError());
 }
 
