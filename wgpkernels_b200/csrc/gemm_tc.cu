@@ -1096,11 +1096,17 @@ struct GemmArgs {
 // Rows a tensor map of a row window may address: the window's position is only known on the GPU.
 constexpr int64_t kUnboundedRows = int64_t(1) << 30;
 
-// Group scales of tiles of up to 128 columns: few rows (a few tiles a CTA) have them gathered by the kernel, a column a lane, instead of regrouped by
-// a launch of their own.  Measured (regrouping and GEMM, L2 cold, regrouped -> gathered, us): exact+g 333 x 12280 x 3008 36.9 -> 35.1, 100 x 4096 x
-// 4096 20.1 -> 17.9, 1024 x 4096 x 4096 44.7 -> 44.5, 2048 x 8192 x 4096 139.4 -> 141.0; block+g 100 x 4096 x 4096 17.7 -> 17.1, 48 x 2048 x 14336
-// 45.5 -> 46.4 (its drain is done with a block sooner than a gather of all columns comes back).
-static bool gathers_scales(const GemmArgs& g, bool hilo) { return g.m <= 1024 && (hilo || g.k <= 8192); }
+// Group scales of tiles of up to 128 columns: few rows have them gathered by the kernel, a column a lane, instead of regrouped by a launch of their
+// own.  That saves the launch, and costs the more the more blocks of K a CTA goes through: block+g is done with a block sooner than a gather of all
+// columns comes back, so it gathers where that is 32 blocks at most; exact+g has the time, until its rows are many or long.  Measured over 7 sizes of
+// weights, 1024 x 1024 to 28672 x 4096 (channels x K), with 33 to 2048 rows, L2 cold, regrouping and GEMM against gathering, us: within the rules
+// 0.3 to 18 % faster (exact+g 333 x 12280 x 3008 35.5 -> 34.0, 33 x 28672 x 4096 47.5 -> 43.3, 1024 x 4096 x 4096 41.7 -> 41.0; block+g 64 x
+// 4096 x 4096 17.5 -> 16.8); beyond them up to a third slower (block+g 333 x 12280 x 3008 31.7 -> 32.7, 1024 x 12280 x 3008 80.4 -> 85.9, 1024 x
+// 5120 x 13824 161 -> 213; exact+g 512 x 5120 x 13824 140 -> 152, 1024 x 8192 x 8192 147.1 -> 149.5, 2048 x 4096 x 4096 76.0 -> 77.7), with exceptions
+// that are left: block+g 200 x 12280 x 3008 33.8 -> 32.1, exact+g 768 x 2048 x 14336 65.0 -> 62.7.
+static bool gathers_scales(const GemmArgs& g, bool hilo, int64_t blocks_of_a_cta) {
+    return g.m <= 1024 && (hilo ? g.k <= 8192 && int64_t(g.m) * g.k <= (1 << 22) : blocks_of_a_cta <= 32);
+}
 
 template <class T, int MODE, int BN, bool WIDE, bool DUMP, int PARTS, bool PAIR = false>
 static int launch(const GemmArgs& g, cudaStream_t stream) {
@@ -1155,8 +1161,9 @@ static int launch(const GemmArgs& g, cudaStream_t stream) {
     p.tiles_n = p.seg_tiles * g.segments;
     p.window = g.window;
     if (S::kWGroup && (!g.scale_scratch || (reinterpret_cast<uintptr_t>(g.scale_scratch) & 15))) return -2;
-    if (S::kWGroup && !(S::kGatherScales && gathers_scales(g, S::kHilo))) {
-        const int kblocks = (g.k + kStageK - 1) / kStageK;
+    const int64_t tiles = int64_t(p.tiles_m) * p.tiles_n;
+    const int sms = g.sms > 0 ? g.sms : 148, kblocks = (g.k + kStageK - 1) / kStageK;
+    if (S::kWGroup && !(S::kGatherScales && gathers_scales(g, S::kHilo, (tiles + sms - 1) / sms * kblocks))) {
         p.n_pad = padded_n(g.n);
         p.sb_blocks = g.scale_scratch;
         const int64_t total = int64_t(kblocks) * p.n_pad;
@@ -1181,8 +1188,6 @@ static int launch(const GemmArgs& g, cudaStream_t stream) {
     if (p.destinations > 1 && !p.tma_y) return -2;  // several destinations are only written by the TMA stores
     if (S::kTmaResidual && p.tma_y && g.residual && !make_output_map(&in_maps.residual, g.residual, g.m, g.n, p.ld_residual, std::is_same<T, bf16>::value, false))
         return int(cudaErrorNotSupported);
-    const int64_t tiles = int64_t(p.tiles_m) * p.tiles_n;
-    const int sms = g.sms > 0 ? g.sms : 148;
     if (PAIR && windowed) return -2;  // a row window's last tile is fetched through a narrower map: single CTAs only
     const int64_t workers = PAIR ? (sms / 2 > 0 ? sms / 2 : 1) : sms;
     cudaLaunchConfig_t config = {};
