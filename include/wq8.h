@@ -116,7 +116,8 @@ int wq8_gemm_at(const int8_t* a, const int8_t* a_lo, const float* sa, const int8
  * accumulation of exact products.  K multiple of 64; x and w 16-byte aligned, ldx a multiple of 8 (-2 otherwise).
  * slots / counters: scratch of the sizes wq8_small_workspace() reports (slots 256-byte aligned); counters zero on entry,
  * left zero.  With scratch and K a multiple of 128 the linear runs on tcgen05 (the activations as INT8 digit planes --
- * see wq8_stream_planes for their accuracy --, K ranges shared over all SMs, partial sums added in a fixed order);
+ * see wq8_stream_planes for their accuracy --, K ranges shared over all SMs, partial sums added in a fixed order), up to four tokens of
+ * long rows and not too many channels on the kernels of wq8_stream_planes, whose digits those are;
  * without scratch (NULL) on the kernels that need none.  The digit split and the stream kernel of a call are launched with
  * programmatic stream serialization: each may start under the tail of the kernel before it on the stream (wq8_transform_rows lets
  * them) and waits for that kernel to finish before it reads what it wrote; callers need to do nothing.
@@ -167,7 +168,9 @@ int wq8_stream_planes(const void* x, int64_t ldx, const int8_t* w, const float* 
  * rows of 2 K, gate | value --, 3 gelu): op(X) is rounded to X's type, as wq8_transform_rows does.  wq8_few_takes() says how a shape runs:
  *   1  one launch, no scratch: up to four tokens, the shapes of wq8_stream_planes whose digit planes fit beside the weights, not rms_norm (every CTA
  *      makes the planes for itself while its first weights are on their way); x 8-byte aligned, ldx a multiple of 4
- *   2  two launches: the other shapes that wq8_small runs on tcgen05, up to 32 tokens; slots and counters of the sizes wq8_small_workspace() reports, both this
+ *   2  two launches, or three: the other shapes that wq8_small runs with scratch, up to 32 tokens (up to four of long rows and not too many
+ *      channels: the input operation by itself, then the kernels of wq8_stream_planes, which are faster there; else on tcgen05, the input
+ *      operation in the digit split); slots and counters of the sizes wq8_small_workspace() reports, both this
  *      call's own until it has run (the counters are cleared by the call itself: no need to hand in zeros); x and
  *      act_weight 16-byte aligned, ldx a multiple of 8
  *   0  not at all (-2 from wq8_few).  w 16-byte aligned.  No counterpart in the reference (which launches the input operation and the product

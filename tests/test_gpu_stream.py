@@ -185,6 +185,30 @@ def test_input_operation_and_stream_in_one_launch(wq, m, shape, act, dtype):
     assert wq.debug_status() == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("act", [None, "rms_norm", "swiglu", "gelu"])
+@pytest.mark.parametrize("m,n,k", [(1, 520, 4096), (3, 1000, 4096 + 128), (4, 264, 14336), (2, 56 * 148, 16384), (4, 56 * 148 + 8, 5120), (3, 112 * 148, 4096), (3, 112 * 148 + 8, 4096),
+                                   (3, 112 * 148, 5120), (3, 112 * 148 + 8, 5120)], ids=str)
+def test_few_tokens_of_long_rows(wq, m, n, k, act, dtype):
+    """Up to four tokens beyond one launch, on both sides of the numbers of channels at which the kernels change: op(x) rounded as transform_rows rounds
+    it, and the oracle's product; wq8_small's bits on those rows where both run the planes; in place; the same bits every time and in both modes."""
+    _, w, sw, bias, res, rs = case(m, n, k, dtype, 171, True)
+    x = randn((m, 2 * k if act == "swiglu" else k), dtype, 172)
+    x[:, ::131] *= 60
+    norm = (1 + 0.1 * randn((k,), torch.float32, 173)).to(dtype) if act == "rms_norm" else None
+    gx, gw, gsw, gbias, gres, grs, gnorm = cuda(x, w, sw, bias, res, rs, norm)
+    prepared = wq.transform_rows(gx, 0, act, gnorm, 1e-6) if act else gx
+    target = gres.clone()
+    y = wq.linear(gx, gw, gsw, gbias, mode="lines", act=act, act_weight=gnorm, eps=1e-6, residual=target, residual_scale=grs, out=target)
+    assert y is target
+    assert rel(y, oracle.weight_only(prepared.cpu(), w.numpy(), sw.numpy(), bias, res, rs, dtype)) < 1e-3
+    assert torch.equal(y, wq.linear(gx, gw, gsw, gbias, mode="small", act=act, act_weight=gnorm, eps=1e-6, residual=gres, residual_scale=grs))
+    if n <= 56 * 148:  # the input operation by itself, then the streams: what linear_prepared() runs
+        ready = wq.prepare(gx, 0, "lines", act, gnorm, 1e-6)
+        assert torch.equal(y, wq.linear_prepared(ready, gw, gsw, gbias, gres, grs))
+    assert not wq._counters[0].any().item() and wq.debug_status() == 0
+
+
 @pytest.mark.parametrize("form", ["linear", "prepared"])
 @pytest.mark.parametrize("m,act", [(1, "rms_norm"), (3, None), (16, "gelu")], ids=str)
 def test_calls_on_several_streams_count_their_own_pieces(wq, m, act, form):

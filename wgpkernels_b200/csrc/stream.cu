@@ -6,7 +6,8 @@
 //   stream_planes  up to 8 tokens: the activations as INT8 digit planes, the weights into mma.sync.m16n8k32.s8 untouched
 //   direct_rows    every other shape and alignment, on plain CUDA cores, with an optional split of K over CTAs
 // stream_few.cu holds the one that does up to 4 tokens and their input operation in one launch (wq8_few, and wq8_stream_planes where the
-// digits of all of K fit beside the weights), and stream_tc.cu the tcgen05 kernel that wq8_small runs with its caller's scratch (up to 32 tokens).
+// digits of all of K fit beside the weights), and stream_tc.cu the tcgen05 kernel that wq8_small runs with its caller's scratch (up to 32 tokens; up to
+// four of long rows and not too many channels on stream_planes).
 // Together they replace w8a16_small / gemv_lines of the reference (wgpkernels/int8/int8_gemm.cu:1039-1151, 1772-1810): same values up
 // to FP32 summation order.
 #include "common.cuh"
@@ -828,8 +829,38 @@ static int64_t tensor_core_scratch(int m, int n, int k, int sms, int64_t* counte
     return bytes && *counter_bytes <= 4096 ? bytes : 0;
 }
 
+// Up to four tokens that are not stream_few's with their input operation: whether the input operation by itself and then the streams of
+// wq8_stream_planes are faster than the tensor-core kernel with the input operation in its digit split.  That kernel spreads every shape over all
+// SMs, and adding up the pieces of shared tiles is most of its time where the channels are few; with many of them it streams better.  The lines lie
+// between the measured sizes (1 to 4 tokens, K of 2048 to 14336, 1024, 4096, 12288 and 28672 channels, device time in a graph, tensor-core kernel and
+// this, us): 3 x 5120 without an operation 12.0 and 6.3 | 12.7 and 9.6 | 19.9 and 18.1 | 31.8 and 32.8; with gelu 12.3 and 8.1 | 12.7 and 11.3 |
+// 19.8 and 20.3 | 31.8 and 35.0; rms_norm in front of stream_few, 1 x 4096, 10.8 and 7.1 | 12.2 and 9.3 | 17.5 and 16.4 | 28.5 and 28.7.
+static bool planes_win(int m, int n, int k, int act, int sms) {
+    if (m > 4 || !wq8_stream_planes_workspace(m, n, k, sms)) return false;
+    const bool one_launch = stream_few_takes(m, k);
+    if (act == kActNone && one_launch) return false;
+    return n <= (act == kActNone || one_launch ? 112 : 56) * (sms > 0 ? sms : 148);
+}
+
+WQ_API int wq8_transform_rows(const void* x, void* out, int m, int k, int64_t ldx, int dtype, int group, int act, const void* act_weight, float eps,
+                              cudaStream_t stream);  // quantize.cu
+
+// scratch: of the size wq8_small_workspace() reports, which holds the rows and the planes of up to four tokens as it holds the digits of eight
+static int planes_in_scratch(const void* x, int64_t ldx, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale, void* y,
+                             int m, int n, int k, int dtype, int act, const void* act_weight, float eps, int sms, void* scratch, cudaStream_t stream) {
+    int8_t* planes = static_cast<int8_t*>(scratch);
+    if (act != kActNone) {
+        const int code = wq8_transform_rows(x, scratch, m, k, ldx, dtype, 0, act, act_weight, eps, stream);
+        if (code) return code;
+        x = scratch;
+        ldx = k;
+        planes += int64_t(kPlaneTokens) * k;  // behind four rows of 16-bit values
+    }
+    return wq8_stream_planes(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, dtype, sms, planes, stream);
+}
+
 // The few-token linear with its input operation: up to four tokens in one launch where the digits of all of K fit beside the weight rings
-// (stream_few.cu; not behind rms_norm, whose row sum comes first), else in two, the input operation being part of the digit split.
+// (stream_few.cu; not behind rms_norm, whose row sum comes first), else in two or three.
 WQ_API int wq8_few_takes(int m, int n, int k, int act, int sms) {
     if (act < kActNone || act > kActGelu) return 0;
     if (m <= 4 && act != kActRms && wq8_stream_planes_workspace(m, n, k, sms) > 0 && stream_few_takes(m, k)) return 1;
@@ -846,7 +877,17 @@ WQ_API int wq8_few(const void* x, int64_t ldx, const int8_t* w, const float* sw,
     if (!form || (reinterpret_cast<uintptr_t>(w) & 15) || (rows & (form == 1 ? 7 : 15))) return -2;
     if (form == 1) return stream_few_launch(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, dtype, act, sms, stream);
     if (!slots || !counters || (reinterpret_cast<uintptr_t>(slots) & 255) || (reinterpret_cast<uintptr_t>(act_weight) & 15)) return -2;
+    if (planes_win(m, n, k, act, sms))
+        return planes_in_scratch(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, dtype, act, act_weight, eps, sms, slots, stream);
     return stream_tc_launch(x, ldx, act, act_weight, eps, w, sw, bias, residual, rscale, y, m, n, k, dtype, sms, slots, counters, stream);
+}
+
+// wq8_small with scratch of its shape
+static int small_in_scratch(const void* x, int64_t ldx, const int8_t* w, const float* sw, const void* bias, const void* residual, const void* rscale, void* y,
+                            int m, int n, int k, int dtype, int sms, float* slots, int* counters, cudaStream_t stream) {
+    if (planes_win(m, n, k, kActNone, sms))
+        return planes_in_scratch(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, dtype, kActNone, nullptr, 0.f, sms, slots, stream);
+    return stream_tc_launch(x, ldx, kActNone, nullptr, 0.f, w, sw, bias, residual, rscale, y, m, n, k, dtype, sms, slots, counters, stream);
 }
 
 WQ_API void wq8_small_workspace(int m, int n, int k, int sms, int64_t* sizes) {
@@ -865,10 +906,10 @@ WQ_API int wq8_small(const void* x, int64_t ldx, const int8_t* w, const float* s
     // every kernel below reads x and w with 16-byte loads (or TMA boxes): unaligned operands are refused, never launched
     if (k <= 0 || k % 64 || m > 32 || ldx % 8 || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(w) & 15)) return -2;
     if (dtype != 0 && dtype != 1) return -1;
-    // with the caller's scratch: the tensor-core kernel (digit planes, stream-K over all SMs)
+    // with the caller's scratch: digit planes, on the tensor-core kernel (stream-K over all SMs) or, a few tokens of long rows, on stream_planes
     int64_t counter_bytes = 0;
     if (slots && counters && (reinterpret_cast<uintptr_t>(slots) & 255) == 0 && tensor_core_scratch(m, n, k, sms, &counter_bytes))
-        return stream_tc_launch(x, ldx, kActNone, nullptr, 0.f, w, sw, bias, residual, rscale, y, m, n, k, dtype, sms, slots, counters, stream);
+        return small_in_scratch(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, dtype, sms, slots, counters, stream);
     const int rows = plan_bulk(m, n, k, sms);
     if (rows && dtype == 0) return launch_bulk<__half>(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, rows, sms, stream);
     if (rows) return launch_bulk<bf16>(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, rows, sms, stream);
@@ -973,7 +1014,7 @@ WQ_API int wq8_small_static(const void* x, int64_t ldx, const int8_t* w, const f
         const cudaError_t cleared = cudaMemsetAsync(counters, 0, size_t(counter_bytes), stream);
         if (cleared != cudaSuccess) return int(cleared);
     }
-    if (tensor_core_bytes) return stream_tc_launch(x, ldx, kActNone, nullptr, 0.f, w, sw, bias, residual, rscale, y, m, n, k, dtype, sms, slots, counters, stream);
+    if (tensor_core_bytes) return small_in_scratch(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, dtype, sms, slots, counters, stream);
     if (rows && dtype == 0) return launch_bulk<__half>(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, rows, sms, stream);
     if (rows) return launch_bulk<bf16>(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, rows, sms, stream);
     if (dtype == 0) return launch_direct<__half>(x, ldx, w, sw, bias, residual, rscale, y, m, n, k, p, slots, counters, stream);
