@@ -40,7 +40,7 @@ def test_quantize_blocks_matches_reference_library(wq, shape, act, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
-@pytest.mark.parametrize("shape", [(37, 1024), (3000, 128), (3001, 1024 - 128), (3000, 1024), (1501, 1024 + 128), (300, 13824), (177, 16384 + 512)], ids=lambda s: f"{s[0]}x{s[1]}")
+@pytest.mark.parametrize("shape", [(37, 1024), (3000, 128), (3001, 1024 - 128), (3000, 1024), (1501, 1024 + 128), (300, 13824), (177, 16384 + 512), (3001, 264), (1500, 1536 + 8)], ids=lambda s: f"{s[0]}x{s[1]}")
 def test_gelu_codes_are_the_accurate_ones(wq, shape, dtype):
     """The block quantizer puts few elements through the accurate gelu; the row quantizer puts all of them.  On rows of one block both have the same
     scale to find, so codes and scales are the same bits: ordinary blocks, blocks without a value above 0.35, zeros, tiny and huge values,

@@ -205,11 +205,12 @@ __global__ void __launch_bounds__(256, 5) quantize_blocks_gelu(const T* __restri
         }
         return;
     }
-    const float amax = gelu_tanh(block_largest), block_inv = 127.f / amax;
+    const float amax = gelu_tanh(block_largest), block_inv = block < kblocks ? 127.f / amax : 0.f;  // (0: what lies past K takes no accurate path)
     if ((lane & 3) == 0 && block < kblocks) scale[row * kblocks + block] = amax / 127.f;
     int8_t* dst = q + row * k + first + lane * 8;
 #pragma unroll
     for (int c = 0; c < kGeluChunks; ++c) {
+        if (first + c * kChunk >= k) break;
         const float inv = __shfl_sync(0xffffffffu, block_inv, (lane & 16) | (c << 2));
         const float2 inverse = make_float2(inv, inv);
         float2 x2[4], t[4], sum[4];
