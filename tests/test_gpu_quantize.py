@@ -119,6 +119,34 @@ def test_rotated_codes_match_oracle(wq, k, group, dtype):
     assert torch.equal(spare, hi)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])
+@pytest.mark.parametrize("group", [16, 64, 256])
+@pytest.mark.parametrize("k", [256, 512, 768 + 64, 1024 + 256, 2048, 13824])
+def test_rotated_rows_in_many_and_in_few(wq, k, group, dtype):
+    """Many rows go to the kernels with sixteen values a lane, a few to those with eight: the same bits, for ordinary values, zeros, tiny and huge ones,
+    infinities and NaN, in chunks that are whole or not and an odd number of them."""
+    k = k // group * group
+    chunks = -(-k // 256)
+    m = max(2049, 60 * 148 // chunks + 3)
+    x = randn((m, k), torch.float32, 34)
+    for i, change in enumerate((lambda v: v * 0, lambda v: v * 1e-7, lambda v: v * 50, lambda v: v * (1e38 if dtype != torch.float16 else 1e3))):
+        x[i::11] = change(x[i::11])
+    x = x.to(dtype)
+    x.view(-1)[5::100003] = float("inf")
+    x.view(-1)[7::100019] = -float("inf")
+    x.view(-1)[9::100043] = float("nan")
+    x = x.cuda()
+    few = max(1, min(64, 9 * 148 // chunks))
+    parts = x.split(few)
+    q, s = wq.quantize_blocks(x, group)
+    assert torch.equal(q, torch.cat([wq.quantize_blocks(part, group)[0] for part in parts]))
+    assert torch.equal(s.view(torch.int32), torch.cat([wq.quantize_blocks(part, group)[1] for part in parts]).view(torch.int32))
+    for hilo in (False, True):
+        got = wq.quantize(x, group, hilo)
+        expected = [torch.cat(t) for t in zip(*[[u for u in wq.quantize(part, group, hilo) if u is not None] for part in parts])]
+        assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip([u for u in got if u is not None], expected))
+
+
 @pytest.mark.parametrize("hilo", [False, True])
 @pytest.mark.parametrize("act", ACTS)
 @pytest.mark.parametrize("shape", [(1, 8), (7, 264), (5, 5120), (3, 13824), (2, 16384 + 512)], ids=lambda s: f"{s[0]}x{s[1]}")

@@ -442,27 +442,29 @@ template <bool PLAIN> WQ_DEVICE void codes_of_sixteen(const float2* v, const flo
 }
 
 template <class T, int GROUP>
-__global__ void __launch_bounds__(256) quantize_blocks_rotated(const T* __restrict__ x, int8_t* __restrict__ q, float* __restrict__ scale, int64_t row0, int k,
-                                                               int64_t ldx, RowShift shift) {
+__global__ void __launch_bounds__(256) quantize_blocks_rotated(const T* __restrict__ x, int8_t* __restrict__ q, float* __restrict__ scale, int64_t row0,
+                                                               uint32_t items, int k, int64_t ldx, RowShift shift) {
     __shared__ __align__(16) float turns[16 * kTurnFloats];
     dependents_may_start();
     const int i = threadIdx.x & 15, half = threadIdx.x >> 4;
-    const int base = (blockIdx.x * 16 + half) * kChunk;
-    if (base - (half & 1) * kChunk >= k) return;  // both halves of a warp, or none
+    // an item is a chunk of a row; the items of all rows are numbered through, so that short rows leave no thread idle
+    const uint32_t item = blockIdx.x * 16 + half, chunks = uint32_t(k + kChunk - 1) / kChunk;
+    if (item - (half & 1) >= items) return;  // both halves of a warp, or none
     float* turn = turns + half * kTurnFloats;
-    const int kblocks = (k + kBlockK - 1) / kBlockK;
-    const int64_t row = row0 + blockIdx.y;
+    const int kblocks = (k + kBlockK - 1) / kBlockK, base = int(item % chunks) * kChunk;
+    const int64_t row = row0 + item / chunks;
     const int col = base + 16 * i;
+    const bool inside = item < items && col < k;
     float2 v[8];
     const T* src = first_row(x, ldx, shift) + row * ldx + col;
-    load_sixteen(src, v, col < k);
+    load_sixteen(src, v, inside);
     rotate_sixteen<GROUP, false>(v, turn, i);
     float strict = 0.f;  // absmax, or NaN
 #pragma unroll
     for (int j = 0; j < 8; ++j) strict = magnitude_or_nan(strict, magnitude_or_nan(v[j].x, v[j].y));
     const bool ordinary = __all_sync(0xffffffffu, fabsf(strict) < kHuge);
     if (!std::is_same<T, __half>::value && !ordinary) {
-        load_sixteen(src, v, col < k);
+        load_sixteen(src, v, inside);
         rotate_sixteen<GROUP, true>(v, turn, i);
     }
     // absmax of the chunk's two blocks: lanes 0-7 end with the first block's, lanes 8-15 with the second's.  (In groups of 16 a lane's values
@@ -476,7 +478,7 @@ __global__ void __launch_bounds__(256) quantize_blocks_rotated(const T* __restri
     for (int d = 4; d > 0; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
     const int block = base / kBlockK + (i >> 3);
     const float own_inv = amax > 0.f ? 127.f / amax : 0.f;
-    if ((i & 7) == 0 && block < kblocks) scale[row * kblocks + block] = amax * group_norm<GROUP>() / 127.f;
+    if ((i & 7) == 0 && block < kblocks && item < items) scale[row * kblocks + block] = amax * group_norm<GROUP>() / 127.f;
     float2 inv[2] = {make_float2(own_inv, own_inv), make_float2(own_inv, own_inv)};
     if constexpr (GROUP > 16) {
         const float other = __shfl_xor_sync(0xffffffffu, own_inv, 8);
@@ -485,7 +487,7 @@ __global__ void __launch_bounds__(256) quantize_blocks_rotated(const T* __restri
     uint32_t c[16];
     if (ordinary && __all_sync(0xffffffffu, own_inv < kHuge)) codes_of_sixteen<true>(v, inv, c);
     else codes_of_sixteen<false>(v, inv, c);
-    store_sixteen<GROUP>(c, turn, i, q + row * k + col, col < k);
+    store_sixteen<GROUP>(c, turn, i, q + row * k + col, inside);
 }
 
 // One scale per row: a CTA per row, CPH chunks a half warp (K <= 4096 CPH), as many warps as the row has work for.
@@ -634,6 +636,27 @@ static int persistent_ctas(int64_t warps_of_work) {
     return int(ctas < cap ? (ctas < 1 ? 1 : ctas) : cap);
 }
 
+// A rotation without an input operation: whether the kernel with sixteen values a lane is the faster one.  It needs fewer instructions, but takes longer
+// for one chunk (the turn through shared memory), so where few chunks or rows fill no more than a wave, the kernel with eight values a lane and shuffles
+// stays.  Both measured over K of 512 to 16384 and 1 to 8192 rows, BF16 and FP32, device time in a graph (shuffles and this, us; BF16): blocks
+// of 64, 16 x 5120 1.87 and 2.21 | 128 x 5120 2.43 and 2.55 | 256 x 5120 3.50 and 3.27 | 8192 x 5120 47.7 and 36.0; 8192 x 1024 11.8 and 9.4;
+// rows in groups of 64, 16 x 2048 1.85 and 2.05 | 512 x 2048 2.83 and 2.71 | 16 x 9216 3.36 and 3.07.  hi and lo in groups of 64: 512 x 5120 6.43
+// and 5.78, but where the other kernel's eight warps have the same number of chunks it is faster, 1024 x 8192 10.7 and 11.4, and so it is on long
+// rows while they are few, 256 x 13824 6.9 and 7.8.  hi and lo in groups of 16: two more digits' worth of registers for twelve shuffles, 1560 x 13824
+// 19.9 and 25.0.  FP32, twice the bytes: rows in groups of 64, 8192 x 8192 63.8 and 72.6 | 8192 x 9216 121.8 and 89.8 | 2048 x 1536 6.4 and 6.9.
+template <class T, int GROUP> static bool sixteen_values_win_blocks(int64_t chunks_of_all_rows) {
+    constexpr int kChunksOfAnSm = sizeof(T) == 4 ? (GROUP == 16 ? 60 : GROUP == 64 ? 120 : 24) : GROUP == 256 ? 10 : 22;
+    return chunks_of_all_rows >= kChunksOfAnSm * device_sm_count();
+}
+template <class T, int GROUP, bool HILO> static bool sixteen_values_win_rows(int m, int k) {
+    if (k > 16384) return false;  // (more than a CTA's registers hold)
+    constexpr bool kWide = sizeof(T) == 4;
+    const bool even = (k + kChunk - 1) / kChunk % 8 == 0;
+    if (GROUP == 256) return (m > 128 || k > (HILO ? 4096 : 2048)) && !(kWide && HILO && even && m < 4096);
+    if (!HILO && !kWide) return m > 256 || k > 4096;
+    return !even && !(kWide && k > 1024 && k <= 2048) && m >= (!HILO ? 257 : k <= 12288 ? 512 : 2048);
+}
+
 template <class T, int GROUP, int ACT>
 static int launch_blocks(const void* x, int8_t* q, float* scale, int m, int k, int64_t ldx, const void* act_weight, float eps, const RowShift& shift,
                          cudaStream_t stream) {
@@ -660,10 +683,19 @@ static int launch_blocks(const void* x, int8_t* q, float* scale, int m, int k, i
                 return int(cudaGetLastError());
             }
         }
+        if constexpr (GROUP > 0 && ACT == kActNone) {
+            if (sixteen_values_win_blocks<T, GROUP>(int64_t(m) * chunks)) {
+                const int64_t most = (int64_t(1) << 30) / chunks;
+                for (int64_t row0 = 0; row0 < m; row0 += most) {
+                    const uint32_t items = uint32_t((m - row0 < most ? m - row0 : most) * chunks);
+                    quantize_blocks_rotated<T, GROUP><<<(items + 15) / 16, 256, 0, stream>>>(src, q, scale, row0, items, k, ldx, shift);
+                }
+                return int(cudaGetLastError());
+            }
+        }
         for (int64_t row0 = 0; row0 < m; row0 += 65535) {
             const dim3 grid((chunks + 7) / 8, unsigned(m - row0 < 65535 ? m - row0 : 65535));
-            if constexpr (GROUP > 0 && ACT == kActNone) quantize_blocks_rotated<T, GROUP><<<dim3((chunks + 15) / 16, grid.y), 256, 0, stream>>>(src, q, scale, row0, k, ldx, shift);
-            else quantize_blocks_items<T, GROUP, ACT><<<grid, 256, 0, stream>>>(src, q, scale, row0, k, ldx, shift);
+            quantize_blocks_items<T, GROUP, ACT><<<grid, 256, 0, stream>>>(src, q, scale, row0, k, ldx, shift);
         }
     }
     return int(cudaGetLastError());
@@ -699,9 +731,9 @@ static int launch_rows(const void* x, int8_t* hi, int8_t* lo, float* scale, int 
     auto src = static_cast<const T*>(x);
     auto aw = static_cast<const T*>(act_weight);
     // (rms_norm: the order of the row's sum is that of eight values a lane; gelu and swiglu: how their last product and the rotation's first sum
-    // are fused is that kernel's; groups of 16 with a low part: two more digits' worth of registers for twelve shuffles, 1560 x 13824 19.9 -> 25.0 us)
+    // are fused is that kernel's)
     if constexpr (GROUP > 0 && ACT == kActNone && !(GROUP == 16 && HILO)) {
-        if (k <= 16384) {
+        if (sixteen_values_win_rows<T, GROUP, HILO>(m, k)) {
             const int chunks = (k + kChunk - 1) / kChunk, per_half = k <= 4096 ? 1 : k <= 8192 ? 2 : 4;
             const int threads = 32 * ((chunks + 2 * per_half - 1) / (2 * per_half));
             if (per_half == 1) quantize_rows_rotated<T, GROUP, HILO, 1><<<m, threads, 0, stream>>>(src, hi, lo, scale, k, ldx, shift);
@@ -709,16 +741,13 @@ static int launch_rows(const void* x, int8_t* hi, int8_t* lo, float* scale, int 
             else quantize_rows_rotated<T, GROUP, HILO, 4><<<m, threads, 0, stream>>>(src, hi, lo, scale, k, ldx, shift);
             return int(cudaGetLastError());
         }
-    } else {
-        auto kernel = quantize_rows<T, GROUP, HILO, ACT, 0>;
-        if (k <= 2048) kernel = quantize_rows<T, GROUP, HILO, ACT, 1>;
-        else if (k <= 4096) kernel = quantize_rows<T, GROUP, HILO, ACT, 2>;
-        else if (k <= 8192) kernel = quantize_rows<T, GROUP, HILO, ACT, 4>;
-        else if (k <= 16384) kernel = quantize_rows<T, GROUP, HILO, ACT, 8>;
-        kernel<<<m, kRowThreads, 0, stream>>>(src, hi, lo, scale, k, ldx, aw, eps, shift);
-        return int(cudaGetLastError());
     }
-    quantize_rows<T, GROUP, HILO, ACT, 0><<<m, kRowThreads, 0, stream>>>(src, hi, lo, scale, k, ldx, aw, eps, shift);  // rotated rows of more than 16384 values
+    auto kernel = quantize_rows<T, GROUP, HILO, ACT, 0>;
+    if (k <= 2048) kernel = quantize_rows<T, GROUP, HILO, ACT, 1>;
+    else if (k <= 4096) kernel = quantize_rows<T, GROUP, HILO, ACT, 2>;
+    else if (k <= 8192) kernel = quantize_rows<T, GROUP, HILO, ACT, 4>;
+    else if (k <= 16384) kernel = quantize_rows<T, GROUP, HILO, ACT, 8>;
+    kernel<<<m, kRowThreads, 0, stream>>>(src, hi, lo, scale, k, ldx, aw, eps, shift);
     return int(cudaGetLastError());
 }
 
