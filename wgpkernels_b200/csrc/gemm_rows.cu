@@ -266,16 +266,21 @@ int gemm_few_rows_cluster(int m, int n, int k, int sms) {
     return 0;
 }
 
-// Whether this kernel is the faster one (against gemm_i8_tc with its own choice of tiles).  Both times are lines in K: gemm_i8_tc brings all of K into
-// one SM, 2.6 ns a value for `exact` and 1.8 for `row`; here a CTA has its share of K, and the exchange costs by the rows.  Fitted in ns to 5 x 8
-// x 6 sizes (17 to 128 rows, 1024 to 9216 channels, K of 512 to 14336) and taken where it wins by a twentieth.  Near the line: `exact`
-// 33 x 3072 x 1024 7.6 and 7.0 us, 128 x 9216 x 4096 16.4 and 17.8 (left alone); `row` 33 x 5120 x 2048 9.5 and 7.9, 128 x 5120 x 4096 12.1 and 12.7.
+// Whether this kernel is the faster one (against gemm_i8_tc, which has tiles of 64 channels for the shapes that fit clusters).  gemm_i8_tc brings all
+// of K into one SM; here a CTA has its share of K, the exchange costs by the rows (the more where a CTA has two blocks of K or fewer to hide
+// its start behind), and all rows go to every CTA; both stream the weights.  In ns, fitted to 9 x 13 x 8 sizes (17 to 128 rows, 512 to 15360 channels, K
+// of 1024 to 14336) and taken where it wins by a twentieth.  Near the line (gemm_i8_tc and this, us): `row` 96 x 9216 x 4096 (rows x channels x K)
+// 13.1 and 14.1, 128 x 5120 x 4096 12.3 and 12.7, 96 x 512 x 1536 6.1 and 6.7 (left alone), 48 x 9216 x 2048 10.8 and 9.1; `exact` 33 x 3072 x
+// 1024 7.6 and 7.0.
 bool gemm_few_rows_wins(int m, int n, int k, bool hilo, int sms) {
-    const int64_t ctas = gemm_few_rows_cluster(m, n, k, sms), slots = (m + 15) / 16 * 16;
+    const int64_t ctas = gemm_few_rows_cluster(m, n, k, sms), slots = (m + 15) / 16 * 16, tiles = (n + kRowsChannels - 1) / kRowsChannels;
     if (!ctas) return false;
-    const int64_t whole = 4400 + (hilo ? 262 : 179) * int64_t(k) / 100;
-    const int64_t split = hilo ? 4600 + 38 * slots + (1700 + 7 * slots) * k / (1000 * ctas) : 5000 + 22 * slots + (1500 + 4 * slots) * k / (1000 * ctas);
-    return 21 * split < 20 * whole;
+    const double kilo = k / 1000., share = kilo / ctas, weights = kilo * n / 1000., copies = double(slots * tiles * ctas) / (sms > 0 ? sms : 148);
+    const double start = k <= 2 * kStageK * ctas ? 5. * slots : 0.;
+    const double whole = hilo ? 4530 + (2490 - 1.4 * m) * kilo + 79.2 * weights : 4370 + (1651 - 1.5 * m) * kilo + 73.5 * weights;
+    const double split = hilo ? 4050 + 29.9 * slots + (1220 + 4.64 * slots) * share + 84.7 * weights + 23.1 * copies
+                              : 3970 + 15.4 * slots + (1234 + 0.75 * slots) * share + 97.9 * weights + 25.5 * copies;
+    return split + start < 0.95 * whole;
 }
 
 template <class T, bool HILO>
