@@ -57,6 +57,11 @@ def test_reads_what_the_kernel_before_it_may_have_written_with_ordinary_loads(na
     assert not re.search(r"__ldg\(|(?<!\w)load_eight\(|ld\.global\.nc", BODIES[name])
 
 
+@pytest.mark.parametrize("name", ["gemm_few_rows", "stream_few"])
+def test_kernels_of_few_rows_and_tokens_read_with_ordinary_loads(name):
+    assert name in launched_early() and not re.search(r"__ldg\(|(?<!\w)load_eight\(|ld\.global\.nc|__restrict__", BODIES[name])
+
+
 @pytest.mark.parametrize("name", sorted(n for n, body in BODIES.items() if "dependents_may_start()" in body))
 def test_lets_the_next_one_start_only_where_everything_before_it_has_finished(name):
     assert "dependency_wait()" in BODIES[name] or name not in launched_early()

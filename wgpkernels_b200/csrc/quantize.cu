@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(256) quantize_blocks_items(const T* __restrict
 //   roundings of t itself, 2.3e-5 for |t| <= 127.  (Below -6, where 1 + tanhf() is 0 or next to it, both are within 1e-9.)
 // One warp takes four chunks of a row: their loads are in flight together, and what is done once per block or per warp (317 instructions a
 // chunk with tanhf, 255 with this arithmetic and a chunk a warp) spreads over more elements.
-// Measured (32760 x 13824, BF16): 556 us with tanhf, 365 so (2.47 and 3.76 TB/s; 1560 x 13824: 29.5 and 22).
+// Measured (32760 x 13824, BF16): 567 us with tanhf, 350 so (2.40 and 3.88 TB/s; 1560 x 13824: 31.0 and 21.5).
 constexpr float kRoundMagic = 12582912.f;  // 1.5 * 2^23: adding it rounds |t| < 2^22 to the nearest even integer, whose low byte is the sum's low byte
 constexpr int kGeluChunks = 4;
 
@@ -347,7 +347,8 @@ __global__ void __launch_bounds__(kRowThreads, CPW > 0 && CPW <= 4 ? 5 : 1) quan
 // through shared memory turns the chunk over, lane i then holds the elements i + 16 j, and the two high digits lie inside a lane as well.
 // (rotate_chunk moves the digits between lanes with 60 shuffles for eight values, one a clock and SM; this takes 20 shared-memory
 // instructions for sixteen.)  The additions are those of rotate_chunk, operand by operand, so the codes are the same.
-// Measured (4096 x 3072, FP16, groups of 256): 20.9 us with the shuffles, 12.7 so; 16384 x 3072: 77 and 47.
+// Measured (one scale a row, groups of 256, alone): 4096 x 3072 22.7 us with the shuffles, 14.4 so (20.5 and 12.6 in a graph); 16384 x 3072 76.6 and 43.9.
+// Few rows take longer this way: the rules at launch_blocks() and launch_rows().
 constexpr int kTurnStride = 20, kTurnFloats = 16 * kTurnStride + 16;  // rows 80 bytes apart, the halves of a warp 16 banks apart: no conflicts
 
 // one digit of sixteen values whose mirrored partners are STEP apart: out[d] = (in0 + in1) + (in2 + in3) - 2 in[3 - d].  HUGE_VALUES: with
@@ -671,8 +672,8 @@ static int launch_blocks(const void* x, int8_t* q, float* scale, int m, int k, i
     } else {
         const int chunks = (k + kChunk - 1) / kChunk;
         if constexpr (ACT == kActGelu && GROUP == 0) {  // (a rotation needs every accurate value)
-            // Four chunks a warp want enough warps: 20 an SM (BF16, 5888 values a row, one chunk a warp with tanhf and this, us: 256 rows 4.0
-            // and 4.5, 512 5.9 and 5.7, 1560 14.0 and 10.9).
+            // Four chunks a warp want enough warps: 20 an SM (BF16, one chunk a warp with tanhf and this, us: 256 rows of 5888 values 4.0 and 4.5,
+            // 512 of 6144 6.2 and 6.1, 1024 of 6144 10.0 and 8.4, 256 of 13824 6.8 and 6.7).
             const int64_t groups = (chunks + kGeluChunks - 1) / kGeluChunks;
             if (m * groups >= 20 * device_sm_count()) {
                 const int64_t most = (int64_t(1) << 30) / groups;

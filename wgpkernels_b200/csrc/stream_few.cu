@@ -17,7 +17,8 @@
 //
 // HBM-bound.  Measured on one token, kernels of a call with a cold L2, input operation + split + stream -> this: 2048 x 2048 (K x N) 5.9 -> 4.1 us,
 // 5120 x 5120 15.2 -> 10, 4096 x 28672 25 -> 24.8, 14336 x 4096 with SwiGLU 18.5 -> 16.5 (a plain read of its weights: 11); MLP of one token,
-// 4096 x 14336, SwiGLU, a pass among others 44.6 -> 40.3 us.
+// 4096 x 14336, SwiGLU, a pass among others 44.6 -> 40.3 us.  With four tokens of 4096 values and some 1000 channels the digits that every CTA makes are most
+// of the time (in a graph 6.3 us, split and stream_planes 5.6; called one by one the second launch costs more than that).
 #include "tc_ptx.cuh"
 
 namespace wq {
@@ -39,7 +40,8 @@ struct FewParams {
     int m, n, k, stages;
 };
 
-// Shared memory: rings, digits (runs, 3 m columns, 128 bytes), column scales (runs, 16 floats), partial sums (2 sets, 16 warps, m, 16 rows + 1), barriers
+// Shared memory: rings, digits (runs, 3 m columns, 128 bytes), column scales (runs, 16 floats), partial sums (kFewSets sets, 16 warps, m,
+// 16 rows + 1), barriers (full: 8 pairs of kFewMaxStages; sums ready, sums free: kFewSets each), the abort flag
 static __host__ __device__ int few_digit_bytes(int m, int k) { return k / kFewRun * 3 * m * kFewRun; }
 static __host__ __device__ int few_scale_bytes(int k) { return k / kFewRun * 16 * 4; }
 static __host__ __device__ int few_partial_bytes(int m) { return kFewSets * kFewWarps * m * (kFewRows + 1) * 4; }
