@@ -224,3 +224,21 @@ def test_few_token_arguments(lib):
     assert call(m=16) == call(m=16, slots=one, counters=one) == call(m=16, slots=scratch) == -2
     assert call(m=16, slots=scratch, counters=one, x=ctypes.c_void_p(8)) == call(m=16, slots=scratch, counters=one, ldx=4100) == -2
     assert call(m=16, slots=scratch, counters=one, act=1, weight=odd) == -2
+
+
+def test_scratch_of_few_tokens_holds_their_rows_and_planes(lib):
+    """Up to four tokens beyond one launch: op(X) in 16 bits and, behind eight bytes a value of K, the planes lie in the scratch that
+    wq8_small_workspace() reports."""
+    lib.wq8_stream_planes_workspace.argtypes, lib.wq8_stream_planes_workspace.restype = [i, i, i, i], i64
+    sizes = (ctypes.c_int64 * 2)()
+    checked = 0
+    for m in (1, 2, 3, 4):
+        for k in (2048, 2048 + 128, 4096 + 128, 5120, 14336, 16384 + 128, 65536):
+            for n in (8, 130, 1000, 16576):
+                for sms in (1, 148, 160):
+                    planes = lib.wq8_stream_planes_workspace(m, n, k, sms)
+                    if planes:
+                        lib.wq8_small_workspace(m, n, k, sms, sizes)
+                        assert 2 * m * k <= 8 * k and 8 * k + planes <= sizes[0] and k * 8 % 256 == 0
+                        checked += 1
+    assert checked > 200
